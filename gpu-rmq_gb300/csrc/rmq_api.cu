@@ -22,7 +22,7 @@ struct rmq_handle {
     const float* d_values = nullptr;
     float* val_buf = nullptr;
     uint32_t* idx_buf = nullptr;
-    uint64_t* idx_buf64 = nullptr;  // 64-bit handles
+    void* tables = nullptr;         // VL: the window tables
     unsigned* counters = nullptr;   // arrival counters of the single-launch build (after the levels)
     bool wide = false;
     uint32_t* err = nullptr;  // invalid-query counter (validate mode)
@@ -32,10 +32,13 @@ struct rmq_handle {
     int with_index = 1;
     int l2_persist = 0;
     int validate = 0;
+    size_t level_bytes = 0;  // device bytes of the levels (CL) or window tables (VL)
     size_t persist_bytes = 0;
     float persist_hit_ratio = 1.f;
     float build_ms = 0.f;
     std::mutex validate_mu;
+
+    bool windows() const { return variant == RMQ_VARIANT_VL || variant == RMQ_VARIANT_VL_SHORT; }
 
     // Staging of the host-buffer calls (rmq_query_host / rmq_query_idx_host),
     // created on the first such call.
@@ -155,9 +158,9 @@ int rmq_debug_bounds_violations(uint64_t* count) {
     if (count == nullptr) return RMQ_ERR_ARG;
     *count = 0;
 #if RMQ_DEBUG_BOUNDS
-    const unsigned int a = rmq::bounds_bad_query(), b = rmq::bounds_bad_batch();
-    if (a == ~0u || b == ~0u) return RMQ_ERR_CUDA;
-    *count = uint64_t(a) + b;
+    const unsigned int a = rmq::bounds_bad_query(), b = rmq::bounds_bad_batch(), c = rmq::bounds_bad_window();
+    if (a == ~0u || b == ~0u || c == ~0u) return RMQ_ERR_CUDA;
+    *count = uint64_t(a) + b + c;
     return RMQ_OK;
 #else
     return RMQ_ERR_UNSUPPORTED;
@@ -232,17 +235,18 @@ int rmq_build(const float* d_values, uint64_t n, const rmq_config* cfg, rmq_stre
 
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     cudaError_t e = cudaSuccess;
-    if (h->lay.num_levels > 1) {
+    if (h->windows()) {
+        h->level_bytes = rmq::window_bytes(n, h->with_index != 0);
+        e = cudaMalloc(&h->tables, h->level_bytes);
+    } else if (h->lay.num_levels > 1) {
         // One allocation: level values, then argmin indices, so that a single
         // L2 access-policy window can cover both.
-        const size_t idx_bytes = h->with_index ? (wide ? sizeof(uint64_t) : sizeof(uint32_t)) : 0;
-        const size_t level_bytes = h->lay.total * (sizeof(float) + idx_bytes);
+        h->level_bytes = h->lay.total * (sizeof(float) + (h->with_index ? sizeof(uint32_t) : 0));
         const size_t counter_bytes = rmq::tail_counters(h->lay) * sizeof(unsigned);
-        e = cudaMalloc(&h->val_buf, level_bytes + counter_bytes);
-        if (e == cudaSuccess && h->with_index && !wide) h->idx_buf = reinterpret_cast<uint32_t*>(h->val_buf + h->lay.total);
-        if (e == cudaSuccess && h->with_index && wide) h->idx_buf64 = reinterpret_cast<uint64_t*>(h->val_buf + h->lay.total);
+        e = cudaMalloc(&h->val_buf, h->level_bytes + counter_bytes);
+        if (e == cudaSuccess && h->with_index) h->idx_buf = reinterpret_cast<uint32_t*>(h->val_buf + h->lay.total);
         if (e == cudaSuccess && counter_bytes > 0) {
-            h->counters = reinterpret_cast<unsigned*>(reinterpret_cast<char*>(h->val_buf) + level_bytes);
+            h->counters = reinterpret_cast<unsigned*>(reinterpret_cast<char*>(h->val_buf) + h->level_bytes);
             e = cudaMemsetAsync(h->counters, 0, counter_bytes, s);
         }
     }
@@ -258,8 +262,8 @@ int rmq_build(const float* d_values, uint64_t n, const rmq_config* cfg, rmq_stre
     if (e == cudaSuccess) e = cudaEventCreate(&e1);
     if (e == cudaSuccess) e = cudaEventRecord(e0, s);
     if (e == cudaSuccess)
-        e = wide ? rmq::launch_build64(h->lay, d_values, h->val_buf, h->idx_buf64, s, h->counters)
-                 : rmq::launch_build(h->lay, d_values, h->val_buf, h->idx_buf, s, h->counters);
+        e = h->windows() ? rmq::launch_window_build(d_values, h->tables, n, h->with_index != 0, wide, s)
+                         : rmq::launch_build(h->lay, d_values, h->val_buf, h->idx_buf, s, h->counters);
     if (e == cudaSuccess) e = cudaEventRecord(e1, s);
     if (e == cudaSuccess) e = cudaEventSynchronize(e1);
     if (e == cudaSuccess) e = cudaEventElapsedTime(&h->build_ms, e0, e1);
@@ -271,12 +275,11 @@ int rmq_build(const float* d_values, uint64_t n, const rmq_config* cfg, rmq_stre
         return cuda_status(e);
     }
 
-    if (h->l2_persist && h->lay.num_levels > 1) {
+    if (h->l2_persist && h->level_bytes > 0) {
         int max_persist = 0, max_window = 0;
         cudaDeviceGetAttribute(&max_persist, cudaDevAttrMaxPersistingL2CacheSize, h->device);
         cudaDeviceGetAttribute(&max_window, cudaDevAttrMaxAccessPolicyWindowSize, h->device);
-        size_t bytes = h->lay.total * (sizeof(float) + (h->idx_buf ? sizeof(uint32_t) : 0) +
-                                       (h->idx_buf64 ? sizeof(uint64_t) : 0));
+        size_t bytes = h->level_bytes;
         if (bytes > size_t(max_window)) bytes = size_t(max_window);
         if (bytes > 0 && max_persist > 0) {
             // Set-aside for persisting lines: the window, up to the device maximum
@@ -299,20 +302,17 @@ static rmq::QueryArgs query_args(const rmq_handle* h, const void* d_lr, uint64_t
                                  void* d_argmin) {
     rmq::QueryArgs a;
     std::memset(&a, 0, sizeof(a));
-    for (uint32_t k = 0; k < h->lay.num_levels; ++k) {
-        const float* val = k == 0 ? h->d_values : h->val_buf + h->lay.offset[k];
-        if (h->wide) {
-            a.lv64.val[k] = val;
-            a.lv64.idx[k] = (k == 0 || h->idx_buf64 == nullptr) ? nullptr : h->idx_buf64 + h->lay.offset[k];
-            a.lv64.size[k] = h->lay.size[k];
-        } else {
-            a.lv.val[k] = val;
+    if (h->windows()) {
+        if (h->wide) a.win64 = rmq::win_view<uint64_t>(h->d_values, h->tables, h->lay.n, h->with_index != 0);
+        else a.win = rmq::win_view<uint32_t>(h->d_values, h->tables, h->lay.n, h->with_index != 0);
+    } else {
+        for (uint32_t k = 0; k < h->lay.num_levels; ++k) {
+            a.lv.val[k] = k == 0 ? h->d_values : h->val_buf + h->lay.offset[k];
             a.lv.idx[k] = (k == 0 || h->idx_buf == nullptr) ? nullptr : h->idx_buf + h->lay.offset[k];
             a.lv.size[k] = uint32_t(h->lay.size[k]);
         }
+        a.lv.num_levels = h->lay.num_levels;
     }
-    a.lv.num_levels = h->lay.num_levels;
-    a.lv64.num_levels = h->lay.num_levels;
     a.wide = h->wide;
     a.q = q;
     a.out_min = d_min;
@@ -326,7 +326,7 @@ static rmq::QueryArgs query_args(const rmq_handle* h, const void* d_lr, uint64_t
     a.variant = h->variant;
     a.lanes = h->lanes;
     a.rf_log = h->lay.rf_log;
-    a.persist_base = h->persist_bytes ? h->val_buf : nullptr;
+    a.persist_base = h->persist_bytes ? (h->windows() ? h->tables : h->val_buf) : nullptr;
     a.persist_bytes = h->persist_bytes;
     a.persist_hit_ratio = h->persist_hit_ratio;
     return a;
@@ -477,6 +477,7 @@ static int query_host_common(const rmq_handle* hc, const void* h_lr, uint64_t q,
         if (e != cudaSuccess) return cuda_status(e);
         std::unique_lock<std::mutex> vlock;
         rmq::QueryArgs a = query_args(h, m_lr, q, static_cast<float*>(m_min), m_idx);
+        a.host_buffers = true;
         uint32_t bad = 0;
         if (h->validate) {
             vlock = std::unique_lock<std::mutex>(h->validate_mu);
@@ -612,9 +613,9 @@ int rmq_get_info(const rmq_handle* h, rmq_info* info) {
     if (h == nullptr || info == nullptr) return RMQ_ERR_ARG;
     fill_info(h->lay, h->variant, h->lanes, info);
     info->index_bits = h->wide ? 64 : 32;
+    // the levels of the plan; a VL handle's window tables take no more
     info->level_bytes = h->lay.num_levels > 1
-                            ? h->lay.total * (sizeof(float) + (h->idx_buf ? sizeof(uint32_t) : 0) +
-                                              (h->idx_buf64 ? sizeof(uint64_t) : 0))
+                            ? h->lay.total * (sizeof(float) + (!h->with_index ? 0 : h->wide ? sizeof(uint64_t) : sizeof(uint32_t)))
                             : 0;
     info->build_ms = h->build_ms;
     return RMQ_OK;
@@ -626,6 +627,7 @@ void rmq_destroy(rmq_handle* h) {
         DeviceGuard guard(h->device);
         free_pipe(h->pipe);
         if (h->val_buf) cudaFree(h->val_buf);
+        if (h->tables) cudaFree(h->tables);
         if (h->err) cudaFree(h->err);
         cudaGetLastError();
     }

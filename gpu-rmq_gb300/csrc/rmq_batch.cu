@@ -2,93 +2,74 @@
 // (include/rmq_gb300_batch.h).
 //
 // Packed layout: every array keeps its values where the caller put them
-// (d_values + value_offsets[a]); all coarse levels of all arrays live in one
-// value buffer and one argmin buffer, array a's levels starting at lvl_base[a]
-// with the single-array layout (src/xxx.h:225-243 rule, rf = 8).  A device
-// descriptor table gives each CTA its array.
+// (d_values + value_offsets[a]); the window tables of all arrays
+// (rmq_window.cuh) live in one buffer, array a's at its descriptor's win_off.
 //
-// Work lists: the build's fused kernel runs one CTA per 8192-entry tile of any
-// array (tile -> array by binary search over tile offsets), a tail kernel one
-// CTA per array; the query kernel one warp per 32 queries of one array.  Build + queries can be captured as one CUDA graph.
+// Work lists: each build kernel runs one CTA per tile of any array, the query
+// kernel one CTA per run of queries of one array.  Build + queries can be
+// captured as one CUDA graph.  384 arrays of 2^10 .. 2^20 values, 1.4e8
+// queries of lognormal(sqrt(size), 1) lengths, build and queries: 4125 us with
+// the block-minimum levels, 2316 us with the tables.
 #include <algorithm>
 #include <cstring>
 #include <new>
 #include <vector>
 
 #include "../../include/rmq_gb300_batch.h"
-#include "rmq_buildk.cuh"
 #include "rmq_internal.h"
-#include "rmq_vl.cuh"
+#include "rmq_window_build.cuh"
 
 namespace rmq {
 
-// Largest a in [0, num) with offs[a] <= x, for non-decreasing offs with
-// offs[0] = 0 <= x < offs[num]; arrays owning no work are skipped.
-__device__ __forceinline__ uint32_t find_owner(const uint64_t* __restrict__ offs, uint32_t num, uint64_t x) {
-    uint32_t lo = 0, hi = num;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (offs[mid] <= x) lo = mid;
-        else hi = mid;
-    }
-    return lo;
+// The build's work lists: entry u of a list is one tile of one array, owner[u]
+// (filled on the device by fill_owner_kernel when the batch is laid out) names
+// the array, so a CTA starts with two dependent loads.
+struct TileList {
+    const uint64_t* off;    // first tile of each array (num_arrays + 1)
+    const uint32_t* owner;  // array of each tile
+};
+
+__device__ __forceinline__ uint64_t batch_tile(const ArrayDesc* descs, const TileList& l, const float* values,
+                                               char* tables, WinOut& w) {
+    const uint32_t a = __ldg(l.owner + blockIdx.x);
+    w = win_out(descs[a], values, tables);
+    return blockIdx.x - __ldg(reinterpret_cast<const unsigned long long*>(l.off) + a);
 }
 
-__device__ __forceinline__ void fill_levelout(const ArrayDesc& d, float* lvl_val, uint32_t* lvl_idx, LevelOut& lo) {
-    for (uint32_t k = 0; k < uint32_t(kMaxLevels); ++k) {
-        const bool has = k > 0 && k < d.num_levels;
-        lo.val[k] = has ? lvl_val + d.lvl_base + d.off[k] : nullptr;
-        lo.idx[k] = (has && lvl_idx != nullptr) ? lvl_idx + d.idx_base + d.off[k] : nullptr;
-        lo.size[k] = k < d.num_levels ? d.size[k] : 0u;
-    }
+__global__ void __launch_bounds__(kBlockThreads)
+batch_block_kernel(const float* __restrict__ values, const ArrayDesc* __restrict__ descs, TileList l, char* tables) {
+    WinOut w;
+    const uint64_t tile = batch_tile(descs, l, values, tables, w);
+    win_block_tile(w, tile);
 }
 
-template <int R>
-__global__ void __launch_bounds__(kFusedThreads)
-batch_fused_kernel(const float* __restrict__ values, const ArrayDesc* __restrict__ descs,
-                   const uint64_t* __restrict__ tile_off, uint32_t num_arrays, float* lvl_val,
-                   uint32_t* lvl_idx) {
-    __shared__ float sv[kTileSectors];
-    __shared__ uint32_t sp[kTileSectors];
-    __shared__ LevelOut lo;
-    __shared__ const float* s_a;
-    __shared__ uint32_t s_n, s_depth, s_tile;
-    if (threadIdx.x == 0) {
-        const uint32_t a = find_owner(tile_off, num_arrays, blockIdx.x);
-        const ArrayDesc& d = descs[a];
-        fill_levelout(d, lvl_val, lvl_idx, lo);
-        s_a = values + d.val_off;
-        s_n = d.size[0];
-        s_tile = uint32_t(blockIdx.x - tile_off[a]);
-        const uint32_t top = d.num_levels - 1u;
-        s_depth = top < fused_depth<R>() ? top : fused_depth<R>();
-    }
-    __syncthreads();
-    if (s_depth > 0) fused_tile<R>(s_a, s_n, lo, s_depth, s_tile, sv, sp);
-}
-
-template <int R>
 __global__ void __launch_bounds__(256)
-batch_tail_kernel(const ArrayDesc* __restrict__ descs, float* lvl_val, uint32_t* lvl_idx) {
-    __shared__ LevelOut lo;
-    __shared__ uint32_t s_from, s_last;
-    if (threadIdx.x == 0) {
-        const ArrayDesc& d = descs[blockIdx.x];
-        fill_levelout(d, lvl_val, lvl_idx, lo);
-        s_last = d.num_levels - 1u;
-        s_from = s_last < fused_depth<R>() ? s_last : fused_depth<R>();
-    }
-    __syncthreads();
-    if (s_from < s_last) tail_levels<R>(lo, s_from, s_last);
+batch_low_kernel(const ArrayDesc* __restrict__ descs, TileList l, char* tables) {
+    __shared__ uint2 sa[kSpan + kHaloLow], sb[kSpan + kHaloLow];
+    WinOut w;
+    const uint64_t tile = batch_tile(descs, l, nullptr, tables, w);
+    win_low_tile(w, tile, sa, sb);
 }
 
-// Work unit of the query kernel: 32 consecutive queries of one array, owned
-// by one warp (a loop over several units per warp made the compiler keep the
-// unit's level pointers in registers: 62-75 instead of 40).  unit_owner[u]
-// (filled on the device by fill_owner_kernel) names the array, so a warp's
-// prologue is two dependent loads; the descriptor is unpacked by 20 lanes at
-// once into the warp's own shared Levels, and no CTA-wide barrier is needed.
-constexpr uint32_t kUnitQueries = 32;
+__global__ void __launch_bounds__(256)
+batch_mid_kernel(const ArrayDesc* __restrict__ descs, TileList l, char* tables) {
+    __shared__ uint2 sa[kSpan + kHaloMid], sb[(kSpan + kHaloMid) / 2];
+    WinOut w;
+    const uint64_t tile = batch_tile(descs, l, nullptr, tables, w);
+    win_mid_tile(w, tile, sa, sb);
+}
+
+__global__ void __launch_bounds__(1024)
+batch_top_kernel(const ArrayDesc* __restrict__ descs, TileList l, char* tables) {
+    WinOut w;
+    batch_tile(descs, l, nullptr, tables, w);
+    win_top(w);
+}
+
+// Work unit of the query kernels: consecutive queries of one array, answered by
+// one CTA (of one request, by one warp, in the served form).  unit_owner[u]
+// (filled on the device by fill_owner_kernel) names the array; one thread
+// unpacks its descriptor into a shared view.
 constexpr uint32_t kMaxQueryThreads = 512;
 
 __global__ void fill_owner_kernel(const uint64_t* __restrict__ unit_off, uint32_t* __restrict__ owner) {
@@ -97,96 +78,53 @@ __global__ void fill_owner_kernel(const uint64_t* __restrict__ unit_off, uint32_
     for (uint64_t u = u0 + threadIdx.x; u < u1; u += blockDim.x) owner[u] = a;
 }
 
-template <int R, bool ARGMIN>
+template <bool ARGMIN>
 __global__ void __launch_bounds__(kMaxQueryThreads)
 batch_query_kernel(const float* __restrict__ values, const ArrayDesc* __restrict__ descs,
                    const uint32_t* __restrict__ unit_owner, const uint64_t* __restrict__ unit_off,
-                   const uint64_t* __restrict__ q_off, uint64_t total_units,
-                   const float* __restrict__ lvl_val, const uint32_t* __restrict__ lvl_idx,
+                   const uint64_t* __restrict__ q_off, const char* __restrict__ tables,
                    const uint2* __restrict__ qs, float* __restrict__ out_min, uint32_t* __restrict__ out_idx) {
-    __shared__ Levels wlv[kMaxQueryThreads / 32];
-    __shared__ uint64_t wq[kMaxQueryThreads / 32][2];
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const uint64_t unit = uint64_t(blockIdx.x) * (blockDim.x >> 5) + warp;
-    if (unit >= total_units) return;  // the whole warp leaves
-    const uint32_t a = __ldg(unit_owner + unit);
-    const ArrayDesc& d = descs[a];
-    Levels& lv = wlv[warp];
-    const uint32_t nl = d.num_levels;
-    if (lane < uint32_t(kMaxLevels)) {
-        const uint32_t k = lane;
-        const bool has = k > 0 && k < nl;
-        lv.val[k] = k == 0 ? values + d.val_off : (has ? lvl_val + d.lvl_base + d.off[k] : nullptr);
-        lv.idx[k] = (has && lvl_idx != nullptr) ? lvl_idx + d.idx_base + d.off[k] : nullptr;
-        lv.size[k] = k < nl ? d.size[k] : 0u;
-    } else if (lane == 31) {
-        lv.num_levels = nl;
-        const uint64_t q0 = q_off[a] + (unit - unit_off[a]) * kUnitQueries;
-        const uint64_t qe = q0 + kUnitQueries;
-        const uint64_t q1 = q_off[a + 1];
-        wq[warp][0] = q0;
-        wq[warp][1] = qe < q1 ? qe : q1;
-    }
-    __syncwarp();
-    const uint32_t cnt = uint32_t(wq[warp][1] - wq[warp][0]);
-    const bool in_range = lane < cnt;
-    uint2 Q = make_uint2(1u, 0u);
-    if (in_range) Q = ld_query(qs + wq[warp][0] + lane);
-    float v;
-    uint32_t idx;
-    const bool valid = vl_compute<R, ARGMIN>(lv, Q, in_range, v, idx);
-    const uint64_t at = wq[warp][0] + lane;  // base re-read after the descent
-    vl_store<ARGMIN>(in_range, valid, v, idx, out_min != nullptr ? out_min + at : nullptr,
-                     ARGMIN ? out_idx + at : nullptr, nullptr);
+    extern __shared__ __align__(16) unsigned char batch_smem[];
+    __shared__ WinView view;
+    const uint32_t a = __ldg(unit_owner + blockIdx.x);
+    if (threadIdx.x == 0) win_load_view(descs[a], values, tables, view);
+    const uint32_t cap = blockDim.x * kBatchLaneQueries;
+    const uint64_t at = q_off[a] + (blockIdx.x - unit_off[a]) * cap;
+    const uint64_t left = q_off[a + 1] - at;
+    const WinLists<uint32_t> sm = win_lists<uint32_t>(batch_smem, cap);
+    __syncthreads();
+    win_block<ARGMIN, kBatchLaneQueries>(view, sm, blockDim.x, qs + at, left < cap ? uint32_t(left) : cap,
+                                         out_min != nullptr ? out_min + at : nullptr, ARGMIN ? out_idx + at : nullptr);
 }
 
 // The served batch's kernel: as batch_query_kernel, but every entry (a
 // request) reads its queries and writes its results through its own ServeIO
 // (staging buffers or the request's page-locked host buffers), and counts
 // its invalid queries so the host needs no pass over the results.
-template <int R>
 __global__ void __launch_bounds__(kMaxQueryThreads)
 serve_query_kernel(const float* __restrict__ values, const ArrayDesc* __restrict__ descs,
                    const uint32_t* __restrict__ unit_owner, const uint64_t* __restrict__ unit_off,
-                   const uint64_t* __restrict__ q_off, uint64_t total_units,
-                   const float* __restrict__ lvl_val, const uint32_t* __restrict__ lvl_idx,
+                   const uint64_t* __restrict__ q_off, uint64_t total_units, const char* __restrict__ tables,
                    const ServeIO* __restrict__ io, uint32_t* __restrict__ bad) {
-    __shared__ Levels wlv[kMaxQueryThreads / 32];
-    __shared__ uint64_t wq[kMaxQueryThreads / 32][2];
+    __shared__ WinView views[kMaxQueryThreads / 32];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint64_t unit = uint64_t(blockIdx.x) * (blockDim.x >> 5) + warp;
     if (unit >= total_units) return;  // the whole warp leaves
     const uint32_t a = __ldg(unit_owner + unit);
-    const ArrayDesc& d = descs[a];
-    Levels& lv = wlv[warp];
-    const uint32_t nl = d.num_levels;
-    if (lane < uint32_t(kMaxLevels)) {
-        const uint32_t k = lane;
-        const bool has = k > 0 && k < nl;
-        lv.val[k] = k == 0 ? values + d.val_off : (has ? lvl_val + d.lvl_base + d.off[k] : nullptr);
-        lv.idx[k] = (has && lvl_idx != nullptr) ? lvl_idx + d.idx_base + d.off[k] : nullptr;
-        lv.size[k] = k < nl ? d.size[k] : 0u;
-    } else if (lane == 31) {
-        lv.num_levels = nl;
-        const uint64_t q0 = (unit - unit_off[a]) * kUnitQueries;  // local to the request
-        const uint64_t qe = q0 + kUnitQueries;
-        const uint64_t q1 = q_off[a + 1] - q_off[a];
-        wq[warp][0] = q0;
-        wq[warp][1] = qe < q1 ? qe : q1;
-    }
-    __syncwarp();
+    if (lane == 0) win_load_view(descs[a], values, tables, views[warp]);
     const ServeIO r = io[a];
-    const uint64_t q0 = wq[warp][0];
-    const uint32_t cnt = uint32_t(wq[warp][1] - q0);
-    const bool in_range = lane < cnt;
+    const uint64_t at = (unit - unit_off[a]) * kServeUnit + lane;  // local to the request
+    const bool in_range = at < q_off[a + 1] - q_off[a];
     uint2 Q = make_uint2(1u, 0u);
-    if (in_range) Q = ld_query(r.qs + q0 + lane);
-    float v;
-    uint32_t idx;
-    const bool valid = vl_compute<R, true>(lv, Q, in_range, v, idx);
+    if (in_range) Q = ld_query(r.qs + at);
+    __syncwarp();
+    const WinView& w = views[warp];
+    const bool valid = in_range && Q.x <= Q.y && Q.y < w.n;
+    WinBest<uint32_t> c{f_nan(), kNoPos, false};
+    if (valid) c = win_one(w, Q.x, Q.y);
     if (in_range) {
-        if (r.out_min != nullptr) st_stream(r.out_min + q0 + lane, v);
-        if (r.out_idx != nullptr) st_stream(r.out_idx + q0 + lane, idx);
+        if (r.out_min != nullptr) st_stream(r.out_min + at, c.v);
+        if (r.out_idx != nullptr) st_stream(r.out_idx + at, win_place(w, c, valid ? Q.x : kNoPos));
     }
     const uint32_t nbad = __popc(__ballot_sync(0xffffffffu, in_range && !valid));
     if (lane == 0 && nbad != 0) atomicAdd(bad + a, nbad);
@@ -196,8 +134,8 @@ cudaError_t launch_serve_query(const ServeQueryArgs& a, cudaStream_t s) {
     if (a.total_units == 0) return cudaSuccess;
     const uint32_t warps = a.threads / 32u;
     const uint32_t grid = uint32_t((a.total_units + warps - 1) / warps);
-    serve_query_kernel<3><<<grid, a.threads, 0, s>>>(a.values, a.descs, a.owner, a.unit_off, a.q_off,
-                                                     a.total_units, a.lvl_val, a.lvl_idx, a.io, a.bad);
+    serve_query_kernel<<<grid, a.threads, 0, s>>>(a.values, a.descs, a.owner, a.unit_off, a.q_off, a.total_units,
+                                                  a.tables, a.io, a.bad);
     return cudaGetLastError();
 }
 
@@ -213,16 +151,13 @@ RMQ_BOUNDS_COUNTER_READER(bounds_bad_batch)
 
 cudaError_t launch_batch_query(const BatchQueryArgs& a, cudaStream_t s) {
     if (a.total_units == 0) return cudaSuccess;
-    const uint32_t warps = a.threads / 32u;
-    const uint32_t grid = uint32_t((a.total_units + warps - 1) / warps);
+    const uint32_t grid = uint32_t(a.total_units), smem = win_lists_bytes<uint32_t>(a.threads * kBatchLaneQueries);
     if (a.out_idx != nullptr) {
-        batch_query_kernel<3, true><<<grid, a.threads, 0, s>>>(a.values, a.descs, a.owner, a.unit_off, a.q_off,
-                                                               a.total_units, a.lvl_val, a.lvl_idx, a.qs,
-                                                               a.out_min, a.out_idx);
+        batch_query_kernel<true><<<grid, a.threads, smem, s>>>(a.values, a.descs, a.owner, a.unit_off, a.q_off,
+                                                            a.tables, a.qs, a.out_min, a.out_idx);
     } else {
-        batch_query_kernel<3, false><<<grid, a.threads, 0, s>>>(a.values, a.descs, a.owner, a.unit_off, a.q_off,
-                                                                a.total_units, a.lvl_val, a.lvl_idx, a.qs,
-                                                                a.out_min, nullptr);
+        batch_query_kernel<false><<<grid, a.threads, smem, s>>>(a.values, a.descs, a.owner, a.unit_off, a.q_off,
+                                                             a.tables, a.qs, a.out_min, nullptr);
     }
     return cudaGetLastError();
 }
@@ -230,6 +165,13 @@ cudaError_t launch_batch_query(const BatchQueryArgs& a, cudaStream_t s) {
 }  // namespace rmq
 
 using rmq::ArrayDesc;
+
+// One build kernel's tiles: the first of each array and the array of each.
+struct TileWork {
+    uint64_t* d_off = nullptr;
+    uint32_t* d_owner = nullptr;
+    uint64_t total = 0;
+};
 
 struct rmq_batch {
     const float* d_values = nullptr;
@@ -240,15 +182,13 @@ struct rmq_batch {
     uint32_t qblock = 128;  // threads per CTA of the query kernel (untuned default)
     int with_index = 1;
     int device = 0;
-    // levels
-    float* lvl_val = nullptr;
-    uint32_t* lvl_idx = nullptr;
-    uint64_t lvl_capacity = 0;  // entries
-    uint64_t lvl_used = 0;
+    // tables
+    char* tables = nullptr;
+    uint64_t lvl_capacity = 0;  // level entries of the deepest accepted plan (set_tuning's limit)
+    uint64_t lvl_used = 0;      // level entries of the current plan
     uint32_t max_levels = 1;
     ArrayDesc* d_descs = nullptr;
-    uint64_t* d_tile_off = nullptr;
-    uint64_t total_tiles = 0;
+    TileWork work[4];  // tiles of the block, low, mid and top kernels
     // queries
     std::vector<uint64_t> q_off;
     uint64_t* d_q_off = nullptr;
@@ -303,60 +243,72 @@ void drop_graph(rmq_batch* b) {
     }
 }
 
-// Lays out every array with its size class's threshold tc[class], uploads
-// descriptors and tile offsets.
-int plan(rmq_batch* b, const uint64_t (&tc)[kClasses], cudaStream_t s) {
-    std::vector<ArrayDesc> descs(b->num_arrays);
-    std::vector<uint64_t> tile_off(b->num_arrays + 1, 0);
+// Plans every array's levels with its size class's threshold tc[class] (the
+// plan that rmq_batch_info reports; the tables do not depend on it).
+int plan(rmq_batch* b, const uint64_t (&tc)[kClasses]) {
     uint64_t base = 0;
     uint32_t max_levels = 1;
     for (uint32_t a = 0; a < b->num_arrays; ++a) {
         const rmq::Layout lay = rmq::plan_layout(b->sizes[a], tc[size_class(b->sizes[a])], 3);
-        ArrayDesc& d = descs[a];
-        std::memset(&d, 0, sizeof(d));
-        d.val_off = b->val_off[a];
-        d.lvl_base = base;
-        d.idx_base = base;
-        d.num_levels = lay.num_levels;
-        for (uint32_t k = 0; k < lay.num_levels; ++k) {
-            d.size[k] = uint32_t(lay.size[k]);
-            d.off[k] = k == 0 ? 0u : uint32_t(lay.offset[k]);
-        }
         if (lay.num_levels > 1) base += lay.total;
         max_levels = std::max(max_levels, lay.num_levels);
-        const uint64_t tiles = lay.num_levels > 1 ? (b->sizes[a] + rmq::kTile - 1) / rmq::kTile : 0;
-        tile_off[a + 1] = tile_off[a] + tiles;
     }
     if (base > b->lvl_capacity) return RMQ_ERR_UNSUPPORTED;
-    cudaError_t e = cudaMemcpyAsync(b->d_descs, descs.data(), sizeof(ArrayDesc) * b->num_arrays,
-                                    cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(b->d_tile_off, tile_off.data(), sizeof(uint64_t) * (b->num_arrays + 1),
-                            cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // tile_off dies here; descs are kept
-    if (e != cudaSuccess) return status_of(e);
-    b->h_descs.swap(descs);
     for (int c = 0; c < kClasses; ++c) b->tc[c] = tc[c];
     b->t = tc[kClasses - 1];
-    b->lvl_used = base;
     b->max_levels = max_levels;
-    b->total_tiles = tile_off[b->num_arrays];
-    drop_graph(b);
+    b->lvl_used = base;
     return RMQ_OK;
 }
 
-int plan(rmq_batch* b, uint64_t t, cudaStream_t s) {
+// Lays out every array's tables, allocates them and uploads the descriptors
+// and the build kernels' work lists (once, at creation).
+int lay_out(rmq_batch* b, cudaStream_t s) {
+    std::vector<uint64_t> off[4];
+    for (auto& o : off) o.assign(b->num_arrays + 1, 0);
+    b->h_descs.resize(b->num_arrays);
+    uint64_t bytes = 0;
+    for (uint32_t a = 0; a < b->num_arrays; ++a) {
+        const rmq::WinShape w = rmq::win_shape(b->sizes[a], b->with_index != 0);
+        b->h_descs[a] = rmq::win_desc(b->val_off[a], bytes, w);
+        bytes += w.bytes;
+        const rmq::WinTiles t = rmq::win_tiles(w);
+        const uint64_t tiles[4] = {t.block, t.low, t.mid, t.top};
+        for (int i = 0; i < 4; ++i) off[i][a + 1] = off[i][a] + tiles[i];
+    }
+    cudaError_t e = cudaMalloc(&b->tables, bytes);
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_descs, sizeof(ArrayDesc) * b->num_arrays);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(b->d_descs, b->h_descs.data(), sizeof(ArrayDesc) * b->num_arrays, cudaMemcpyHostToDevice, s);
+    for (int i = 0; i < 4 && e == cudaSuccess; ++i) {
+        TileWork& w = b->work[i];
+        w.total = off[i][b->num_arrays];
+        if (w.total == 0) continue;
+        if (w.total > 0x7FFFFFFFull) return RMQ_ERR_UNSUPPORTED;  // one CTA per tile
+        e = cudaMalloc(&w.d_off, sizeof(uint64_t) * (b->num_arrays + 1));
+        if (e == cudaSuccess) e = cudaMalloc(&w.d_owner, sizeof(uint32_t) * w.total);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(w.d_off, off[i].data(), sizeof(uint64_t) * (b->num_arrays + 1), cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess) e = rmq::launch_fill_owner(w.d_off, b->num_arrays, w.d_owner, s);
+    }
+    const cudaError_t es = cudaStreamSynchronize(s);  // the host lists die here
+    return status_of(e != cudaSuccess ? e : es);
+}
+
+int plan(rmq_batch* b, uint64_t t) {
     const uint64_t tc[kClasses] = {t, t, t};
-    return plan(b, tc, s);
+    return plan(b, tc);
 }
 
 int upload_blocks(rmq_batch* b, cudaStream_t s) {
     std::vector<uint64_t> blk(b->num_arrays + 1, 0);
     for (uint32_t a = 0; a < b->num_arrays; ++a) {
         const uint64_t qa = b->q_off[a + 1] - b->q_off[a];
-        blk[a + 1] = blk[a] + (qa + rmq::kUnitQueries - 1) / rmq::kUnitQueries;
+        const uint64_t unit = uint64_t(b->qblock) * rmq::kBatchLaneQueries;
+        blk[a + 1] = blk[a] + (qa + unit - 1) / unit;
     }
     const uint64_t units = blk[b->num_arrays];
+    if (units > 0x7FFFFFFFull) return RMQ_ERR_UNSUPPORTED;  // one CTA per unit
     cudaError_t e = cudaSuccess;
     if (units > b->owner_capacity) {
         if (b->d_owner != nullptr) cudaFree(b->d_owner);
@@ -377,16 +329,14 @@ int upload_blocks(rmq_batch* b, cudaStream_t s) {
 }
 
 cudaError_t enqueue_build(rmq_batch* b, cudaStream_t s) {
-    if (b->total_tiles == 0) return cudaSuccess;
-    rmq::batch_fused_kernel<3><<<uint32_t(b->total_tiles), rmq::kFusedThreads, 0, s>>>(
-        b->d_values, b->d_descs, b->d_tile_off, b->num_arrays, b->lvl_val, b->lvl_idx);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    if (b->max_levels - 1 > rmq::fused_depth<3>()) {
-        rmq::batch_tail_kernel<3><<<b->num_arrays, 256, 0, s>>>(b->d_descs, b->lvl_val, b->lvl_idx);
-        e = cudaGetLastError();
-    }
-    return e;
+    const TileWork* w = b->work;
+    const auto list = [&](int i) { return rmq::TileList{w[i].d_off, w[i].d_owner}; };
+    rmq::batch_block_kernel<<<uint32_t(w[0].total), rmq::kBlockThreads, 0, s>>>(b->d_values, b->d_descs, list(0),
+                                                                               b->tables);
+    if (w[1].total > 0) rmq::batch_low_kernel<<<uint32_t(w[1].total), 256, 0, s>>>(b->d_descs, list(1), b->tables);
+    if (w[2].total > 0) rmq::batch_mid_kernel<<<uint32_t(w[2].total), 256, 0, s>>>(b->d_descs, list(2), b->tables);
+    if (w[3].total > 0) rmq::batch_top_kernel<<<uint32_t(w[3].total), 1024, 0, s>>>(b->d_descs, list(3), b->tables);
+    return cudaGetLastError();
 }
 
 cudaError_t enqueue_query(rmq_batch* b, cudaStream_t s) {
@@ -397,8 +347,7 @@ cudaError_t enqueue_query(rmq_batch* b, cudaStream_t s) {
     a.unit_off = b->d_blk_off;
     a.q_off = b->d_q_off;
     a.total_units = b->total_blocks;
-    a.lvl_val = b->lvl_val;
-    a.lvl_idx = b->lvl_idx;
+    a.tables = b->tables;
     a.qs = reinterpret_cast<const uint2*>(b->d_lr);
     a.out_min = b->d_min;
     a.out_idx = b->d_argmin;
@@ -456,19 +405,14 @@ int rmq_batch_create(const float* d_values, const uint64_t* value_offsets, const
     b->lvl_capacity = cap;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     cudaError_t e = cudaSuccess;
-    if (cap > 0) {
-        e = cudaMalloc(&b->lvl_val, cap * sizeof(float));
-        if (e == cudaSuccess && b->with_index) e = cudaMalloc(&b->lvl_idx, cap * sizeof(uint32_t));
-    }
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_descs, sizeof(ArrayDesc) * num_arrays);
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_tile_off, sizeof(uint64_t) * (num_arrays + 1));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_q_off, sizeof(uint64_t) * (num_arrays + 1));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_blk_off, sizeof(uint64_t) * (num_arrays + 1));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->cap_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreate(&b->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&b->ev1);
     int st = status_of(e);
-    if (st == RMQ_OK) st = plan(b, t, s);
+    if (st == RMQ_OK) st = plan(b, t);
+    if (st == RMQ_OK) st = lay_out(b, s);
     if (st != RMQ_OK) {
         rmq_batch_destroy(b);
         return st;
@@ -555,28 +499,20 @@ int rmq_batch_run_per_array(rmq_batch* b, rmq_stream_t stream) {
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     for (uint32_t a = 0; a < b->num_arrays; ++a) {
         const ArrayDesc& d = b->h_descs[a];
-        const rmq::Layout lay = rmq::plan_layout(b->sizes[a], b->tc[size_class(b->sizes[a])], 3);
         const float* vals = b->d_values + d.val_off;
-        float* lvl = b->lvl_val + d.lvl_base;
-        uint32_t* idx = b->lvl_idx != nullptr ? b->lvl_idx + d.idx_base : nullptr;
-        cudaError_t e = rmq::launch_build(lay, vals, lvl, idx, s);
+        char* tables = b->tables + d.win_off;
+        cudaError_t e = rmq::launch_window_build(vals, tables, b->sizes[a], b->with_index != 0, false, s);
         if (e != cudaSuccess) return status_of(e);
         const uint64_t q0 = b->q_off[a], q = b->q_off[a + 1] - q0;
         if (q == 0) continue;
         rmq::QueryArgs qa;
         std::memset(&qa, 0, sizeof(qa));
-        for (uint32_t k = 0; k < lay.num_levels; ++k) {
-            qa.lv.val[k] = k == 0 ? vals : lvl + lay.offset[k];
-            qa.lv.idx[k] = (k == 0 || idx == nullptr) ? nullptr : idx + lay.offset[k];
-            qa.lv.size[k] = uint32_t(lay.size[k]);
-        }
-        qa.lv.num_levels = lay.num_levels;
+        qa.win = rmq::win_view<uint32_t>(vals, tables, b->sizes[a], b->with_index != 0);
         qa.qs = reinterpret_cast<const uint2*>(b->d_lr) + q0;
         qa.q = q;
         qa.out_min = b->d_min != nullptr ? b->d_min + q0 : nullptr;
         qa.out_idx = b->d_argmin != nullptr ? b->d_argmin + q0 : nullptr;
         qa.variant = RMQ_VARIANT_VL;
-        qa.lanes = 8;
         qa.rf_log = 3;
         e = rmq::launch_query(qa, s);
         if (e != cudaSuccess) return status_of(e);
@@ -604,59 +540,32 @@ int rmq_batch_autotune(rmq_batch* b, rmq_stream_t stream, rmq_batch_info* info) 
     if (b == nullptr || !b->queries_set) return RMQ_ERR_ARG;
     DeviceGuard guard(b->device);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    // 1. one threshold for every array x CTA size
-    float best = -1.f;
-    uint64_t best_t = b->t;
-    uint32_t best_block = b->qblock;
-    for (uint64_t t : kTuneT) {
-        int st = plan(b, t, s);
-        if (st != RMQ_OK) return st;
-        cudaError_t e = enqueue_build(b, s);
-        if (e != cudaSuccess) return status_of(e);
-        for (uint32_t qb : kTuneBlock) {
-            b->qblock = qb;
-            st = upload_blocks(b, s);
-            if (st != RMQ_OK) return st;
-            float ms = 0.f;
-            st = time_query(b, s, 2, &ms);
-            if (st != RMQ_OK) return st;
-            if (best < 0.f || ms < best) {
-                best = ms;
-                best_t = t;
-                best_block = qb;
-            }
-        }
+    uint64_t tc[kClasses];
+    for (int c = 0; c < kClasses; ++c) {
+        const uint64_t* end = kTuneT + sizeof(kTuneT) / sizeof(kTuneT[0]);
+        tc[c] = std::find(kTuneT, end, b->tc[c]) != end ? b->tc[c] : kBatchDefaultT;
     }
-    // 2. each size class's threshold in turn (largest arrays first, they
-    // carry most of the queries), the others held; a change is kept only
-    // when it is faster by more than 0.5 %, above the timing noise.
-    b->qblock = best_block;
-    int st = upload_blocks(b, s);
-    if (st != RMQ_OK) return st;
-    uint64_t best_tc[kClasses] = {best_t, best_t, best_t};
-    for (int c = kClasses - 1; c >= 0; --c) {
-        for (uint64_t t : kTuneT) {
-            if (t == best_tc[c]) continue;
-            uint64_t tc[kClasses] = {best_tc[0], best_tc[1], best_tc[2]};
-            tc[c] = t;
-            st = plan(b, tc, s);
-            if (st != RMQ_OK) return st;
-            cudaError_t e = enqueue_build(b, s);
-            if (e != cudaSuccess) return status_of(e);
-            float ms = 0.f;
-            st = time_query(b, s, 2, &ms);
-            if (st != RMQ_OK) return st;
-            if (ms < best * 0.995f) {
-                best = ms;
-                best_tc[c] = t;
-            }
-        }
-    }
-    st = plan(b, best_tc, s);
+    int st = plan(b, tc);
     if (st != RMQ_OK) return st;
     cudaError_t e = enqueue_build(b, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return status_of(e);
+    float best = -1.f;
+    uint32_t best_block = b->qblock;
+    for (uint32_t qb : kTuneBlock) {
+        b->qblock = qb;
+        st = upload_blocks(b, s);
+        if (st != RMQ_OK) return st;
+        float ms = 0.f;
+        st = time_query(b, s, 2, &ms);
+        if (st != RMQ_OK) return st;
+        if (best < 0.f || ms < best) {
+            best = ms;
+            best_block = qb;
+        }
+    }
+    b->qblock = best_block;
+    st = upload_blocks(b, s);
+    if (st != RMQ_OK) return st;
     b->build_timed = false;
     b->query_ms = best;
     return info != nullptr ? rmq_batch_get_info(b, info) : RMQ_OK;
@@ -667,15 +576,14 @@ int rmq_batch_set_tuning(rmq_batch* b, uint64_t scan_threshold, uint32_t query_b
         query_block % 32 != 0)
         return RMQ_ERR_ARG;
     DeviceGuard guard(b->device);
-    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    int st = plan(b, scan_threshold, s);  // RMQ_ERR_UNSUPPORTED when the levels would not fit
+    int st = plan(b, scan_threshold);  // RMQ_ERR_UNSUPPORTED when the levels would not fit
     if (st != RMQ_OK) return st;
     b->qblock = query_block;
+    drop_graph(b);
     if (b->queries_set) {
-        st = upload_blocks(b, s);
+        st = upload_blocks(b, reinterpret_cast<cudaStream_t>(stream));
         if (st != RMQ_OK) return st;
     }
-    drop_graph(b);
     b->build_timed = false;
     return RMQ_OK;
 }
@@ -691,15 +599,14 @@ int rmq_batch_set_class_tuning(rmq_batch* b, const uint64_t* class_thresholds, u
         tc[c] = class_thresholds[c];
     }
     DeviceGuard guard(b->device);
-    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    int st = plan(b, tc, s);  // RMQ_ERR_UNSUPPORTED when the levels would not fit
+    int st = plan(b, tc);  // RMQ_ERR_UNSUPPORTED when the levels would not fit
     if (st != RMQ_OK) return st;
     b->qblock = query_block;
+    drop_graph(b);
     if (b->queries_set) {
-        st = upload_blocks(b, s);
+        st = upload_blocks(b, reinterpret_cast<cudaStream_t>(stream));
         if (st != RMQ_OK) return st;
     }
-    drop_graph(b);
     b->build_timed = false;
     return RMQ_OK;
 }
@@ -710,7 +617,7 @@ int rmq_batch_get_info(const rmq_batch* bc, rmq_batch_info* info) {
     std::memset(info, 0, sizeof(*info));
     info->num_arrays = b->num_arrays;
     for (uint64_t n : b->sizes) info->total_values += n;
-    info->level_bytes = b->lvl_used * (sizeof(float) + (b->lvl_idx ? sizeof(uint32_t) : 0));
+    info->level_bytes = b->lvl_used * (sizeof(float) + (b->with_index ? sizeof(uint32_t) : 0));
     info->scan_threshold = b->t;
     info->query_block = b->qblock;
     info->max_levels = b->max_levels;
@@ -737,10 +644,12 @@ void rmq_batch_destroy(rmq_batch* b) {
         if (b->cap_stream) cudaStreamDestroy(b->cap_stream);
         if (b->ev0) cudaEventDestroy(b->ev0);
         if (b->ev1) cudaEventDestroy(b->ev1);
-        cudaFree(b->lvl_val);
-        cudaFree(b->lvl_idx);
+        cudaFree(b->tables);
         cudaFree(b->d_descs);
-        cudaFree(b->d_tile_off);
+        for (TileWork& w : b->work) {
+            cudaFree(w.d_off);
+            cudaFree(w.d_owner);
+        }
         cudaFree(b->d_q_off);
         cudaFree(b->d_blk_off);
         cudaFree(b->d_owner);

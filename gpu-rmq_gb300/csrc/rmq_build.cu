@@ -28,25 +28,24 @@ __device__ __forceinline__ void wait_previous_grid() { asm volatile("griddepcont
 // wait_previous_grid until this grid completes).
 __device__ __forceinline__ void allow_next_grid() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// One output block per group of LPB = rf/8 lanes (P: position type).
+// One output block per group of LPB = rf/8 lanes .
 //   src, src_size : level k (level 0 = caller's array, not padded)
 //   src_idx       : level-0 indices of level k's entries (null for k = 0)
 //   src_padded    : src has at least round_up(src_size, 8) readable entries
-template <int R, typename P>
+template <int R>
 __global__ void __launch_bounds__(256)
-build_step_kernel(const float* __restrict__ src, const P* __restrict__ src_idx, P src_size, int src_padded,
-                  float* __restrict__ dst, P* __restrict__ dst_idx, P dst_size) {
+build_step_kernel(const float* __restrict__ src, const uint32_t* __restrict__ src_idx, uint32_t src_size, int src_padded,
+                  float* __restrict__ dst, uint32_t* __restrict__ dst_idx, uint32_t dst_size) {
     constexpr uint32_t LPB = (1u << R) / 8u;
-    constexpr P kNone = IdxTraits<P>::none;
-    wait_previous_grid();
+        wait_previous_grid();
     allow_next_grid();
     const uint64_t gt = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    const P blk = P(gt / LPB);
+    const uint32_t blk = uint32_t(gt / LPB);
     const uint32_t sub = uint32_t(gt % LPB);
 
-    VPT<P> c{f_inf(), kNone};
+    VP c{f_inf(), kNoPos};
     if (blk < dst_size) {
-        const P s = (blk << R) + 8u * sub;
+        const uint32_t s = (blk << R) + 8u * sub;
         if (s < src_size) {
             float v[8];
             if (src_padded || s + 8u <= src_size) {
@@ -57,7 +56,7 @@ build_step_kernel(const float* __restrict__ src, const P* __restrict__ src_idx, 
             }
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                if (s + j < src_size) vp_take(c, v[j], src_idx != nullptr ? __ldg(src_idx + s + j) : P(s + j));
+                if (s + j < src_size) vp_take(c, v[j], src_idx != nullptr ? __ldg(src_idx + s + j) : uint32_t(s + j));
             }
         }
     }
@@ -66,8 +65,8 @@ build_step_kernel(const float* __restrict__ src, const P* __restrict__ src_idx, 
 #pragma unroll
     for (uint32_t o = 1; o < LPB; o <<= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, c.v, o);
-        const P op = __shfl_xor_sync(0xffffffffu, c.p, o);
-        if (op != kNone && (c.p == kNone || ov < c.v || (ov == c.v && op < c.p))) {
+        const uint32_t op = __shfl_xor_sync(0xffffffffu, c.p, o);
+        if (op != kNoPos && (c.p == kNoPos || ov < c.v || (ov == c.v && op < c.p))) {
             c.v = ov;
             c.p = op;
         }
@@ -110,18 +109,18 @@ Layout plan_layout(uint64_t n, uint64_t t, uint32_t rf_log) {
 // The levels above are small; a single-CTA tail kernel finishes them (or
 // grid-wide build_step launches while they are still large).
 // ---------------------------------------------------------------------------
-template <int R, typename P>
+template <int R>
 __global__ void __launch_bounds__(kFusedThreads)
-build_fused_kernel(const float* __restrict__ a, P n, LevelOutT<P> out, uint32_t depth, TailPlan tp) {
+build_fused_kernel(const float* __restrict__ a, uint32_t n, LevelOut out, uint32_t depth, TailPlan tp) {
     __shared__ float sv[kTileSectors];
-    __shared__ P sp[kTileSectors];
+    __shared__ uint32_t sp[kTileSectors];
     allow_next_grid();
     fused_tile<R>(a, n, out, depth, blockIdx.x, sv, sp);
     if (tp.top > tp.depth) tail_upward<R>(out, tp, blockIdx.x);
 }
 
-template <int R, typename P>
-__global__ void __launch_bounds__(1024) build_tail_kernel(LevelOutT<P> out, uint32_t from, uint32_t last) {
+template <int R>
+__global__ void __launch_bounds__(1024) build_tail_kernel(LevelOut out, uint32_t from, uint32_t last) {
     wait_previous_grid();
     tail_levels<R>(out, from, last);
 }
@@ -185,19 +184,19 @@ uint64_t tail_counters(const Layout& lay) {
     return c;
 }
 
-template <int R, typename P>
-static cudaError_t build_levels(const Layout& lay, const float* d_values, float* val_buf, P* idx_buf,
+template <int R>
+static cudaError_t build_levels(const Layout& lay, const float* d_values, float* val_buf, uint32_t* idx_buf,
                                 cudaStream_t s, unsigned* counters) {
     constexpr uint32_t LPB = (1u << R) / 8u;
     if (lay.num_levels < 2) return cudaSuccess;
-    LevelOutT<P> out;
+    LevelOut out;
     for (uint32_t k = 0; k < uint32_t(kMaxLevels); ++k) {
         out.val[k] = nullptr;
         out.idx[k] = nullptr;
         out.size[k] = 0;
     }
     for (uint32_t k = 0; k < lay.num_levels; ++k) {
-        out.size[k] = P(lay.size[k]);
+        out.size[k] = uint32_t(lay.size[k]);
         if (k > 0) {
             out.val[k] = val_buf + lay.offset[k];
             out.idx[k] = idx_buf == nullptr ? nullptr : idx_buf + lay.offset[k];
@@ -206,7 +205,7 @@ static cudaError_t build_levels(const Layout& lay, const float* d_values, float*
     uint32_t fused, steps;
     bool tail;
     plan_launches<R>(lay, &fused, &steps, &tail);
-    const P n = P(lay.size[0]);
+    const uint32_t n = uint32_t(lay.size[0]);
     const uint32_t tiles = uint32_t((uint64_t(n) + kTile - 1) / kTile);
     TailPlan tp = {};
     tp.depth = fused;
@@ -221,43 +220,32 @@ static cudaError_t build_levels(const Layout& lay, const float* d_values, float*
             c += lay.size[k];
         }
     }
-    build_fused_kernel<R, P><<<tiles, kFusedThreads, 0, s>>>(d_values, n, out, fused, tp);
+    build_fused_kernel<R><<<tiles, kFusedThreads, 0, s>>>(d_values, n, out, fused, tp);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || tp.top > tp.depth) return e;
     uint32_t k = fused;
     for (uint32_t i = 0; i < steps; ++i, ++k) {
-        const P dst_size = out.size[k + 1];
+        const uint32_t dst_size = out.size[k + 1];
         const uint64_t threads = uint64_t(dst_size) * LPB;
         const uint32_t grid = uint32_t((threads + 255) / 256);
-        e = launch_dependent(build_step_kernel<R, P>, grid, 256, s, out.val[k], (const P*)out.idx[k], out.size[k],
+        e = launch_dependent(build_step_kernel<R>, grid, 256, s, out.val[k], (const uint32_t*)out.idx[k], out.size[k],
                              1, out.val[k + 1], out.idx[k + 1], dst_size);
         if (e != cudaSuccess) return e;
     }
     if (tail) {
-        e = launch_dependent(build_tail_kernel<R, P>, 1, 1024, s, out, k, lay.num_levels - 1);
+        e = launch_dependent(build_tail_kernel<R>, 1, 1024, s, out, k, lay.num_levels - 1);
     }
     return e;
 }
 
-template <typename P>
-static cudaError_t launch_build_p(const Layout& lay, const float* d_values, float* val_buf, P* idx_buf,
-                                  cudaStream_t s, unsigned* counters) {
-    switch (lay.rf_log) {
-        case 3: return build_levels<3, P>(lay, d_values, val_buf, idx_buf, s, counters);
-        case 4: return build_levels<4, P>(lay, d_values, val_buf, idx_buf, s, counters);
-        case 5: return build_levels<5, P>(lay, d_values, val_buf, idx_buf, s, counters);
-        default: return cudaErrorInvalidValue;
-    }
-}
-
 cudaError_t launch_build(const Layout& lay, const float* d_values, float* val_buf,
                          uint32_t* idx_buf, cudaStream_t s, unsigned* counters) {
-    return launch_build_p<uint32_t>(lay, d_values, val_buf, idx_buf, s, counters);
-}
-
-cudaError_t launch_build64(const Layout& lay, const float* d_values, float* val_buf,
-                           uint64_t* idx_buf, cudaStream_t s, unsigned* counters) {
-    return launch_build_p<uint64_t>(lay, d_values, val_buf, idx_buf, s, counters);
+    switch (lay.rf_log) {
+        case 3: return build_levels<3>(lay, d_values, val_buf, idx_buf, s, counters);
+        case 4: return build_levels<4>(lay, d_values, val_buf, idx_buf, s, counters);
+        case 5: return build_levels<5>(lay, d_values, val_buf, idx_buf, s, counters);
+        default: return cudaErrorInvalidValue;
+    }
 }
 
 }  // namespace rmq

@@ -1,5 +1,4 @@
-// rmq_buildk.cuh — build device functions shared by the single-array build
-// (rmq_build.cu) and the batched build (rmq_batch.cu).
+// rmq_buildk.cuh — device functions of the level build (rmq_build.cu).
 #pragma once
 
 #include "rmq_common.cuh"
@@ -11,27 +10,21 @@ constexpr uint32_t kTileSectors = kTile / 8;
 constexpr uint32_t kFusedThreads = 256;
 constexpr uint32_t kTailMaxEntries = 16384;  // largest level the tail CTA reads
 
-// P: position type (uint32_t, or uint64_t for arrays beyond 2^32 entries).
-template <typename P>
-struct LevelOutT {
+struct LevelOut {
     float* val[kMaxLevels];
-    P* idx[kMaxLevels];  // null entries when argmin arrays are not built
-    P size[kMaxLevels];
+    uint32_t* idx[kMaxLevels];  // null entries when argmin arrays are not built
+    uint32_t size[kMaxLevels];
 };
-using LevelOut = LevelOutT<uint32_t>;
 
 // First-occurrence minimum over candidates visited in ascending position;
-// p == none marks an absent candidate.
-template <typename P>
-struct VPT {
+// p == kNoPos marks an absent candidate.
+struct VP {
     float v;
-    P p;
+    uint32_t p;
 };
 
-template <typename P>
-__device__ __forceinline__ void vp_take(VPT<P>& cur, float v, P p) {
-    constexpr P kNone = IdxTraits<P>::none;
-    if (p != kNone && (cur.p == kNone || v < cur.v)) {
+__device__ __forceinline__ void vp_take(VP& cur, float v, uint32_t p) {
+    if (p != kNoPos && (cur.p == kNoPos || v < cur.v)) {
         cur.v = v;
         cur.p = p;
     }
@@ -45,11 +38,9 @@ __host__ __device__ constexpr uint32_t fused_depth() {
 // One CTA of kFusedThreads threads builds levels 1..depth of `tile` (entries
 // [tile * kTile, (tile + 1) * kTile) of level 0); sv / sp are kTileSectors
 // entries of shared memory.
-template <int R, typename P>
-__device__ __forceinline__ void fused_tile(const float* __restrict__ a, P n, const LevelOutT<P>& out,
-                                           uint32_t depth, uint64_t tile, float* sv, P* sp) {
-    using VP = VPT<P>;
-    constexpr P kNone = IdxTraits<P>::none;
+template <int R>
+__device__ __forceinline__ void fused_tile(const float* __restrict__ a, uint32_t n, const LevelOut& out,
+                                           uint32_t depth, uint64_t tile, float* sv, uint32_t* sp) {
     constexpr uint32_t RF = 1u << R;
     constexpr uint32_t SPB = RF / 8u;  // sectors per level-1 block
     const uint32_t tid = threadIdx.x;
@@ -81,14 +72,14 @@ __device__ __forceinline__ void fused_tile(const float* __restrict__ a, P n, con
                 }
             }
             sv[sec] = mv;
-            sp[sec] = P(base + 8u * sec + j);
+            sp[sec] = uint32_t(base + 8u * sec + j);
         }
     } else {
 #pragma unroll
         for (uint32_t i = 0; i < kSecPer; ++i) {
             const uint32_t sec = tid + kFusedThreads * i;
             const uint64_t s = base + 8u * sec;
-            VP c{f_inf(), kNone};
+            VP c{f_inf(), kNoPos};
             if (s < n) {
                 float v[8];
                 if (s + 8u <= n) {
@@ -99,7 +90,7 @@ __device__ __forceinline__ void fused_tile(const float* __restrict__ a, P n, con
                 }
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
-                    if (s + j < n) vp_take(c, v[j], P(s + j));
+                    if (s + j < n) vp_take(c, v[j], uint32_t(s + j));
             }
             sv[sec] = c.v;
             sp[sec] = c.p;
@@ -118,7 +109,7 @@ __device__ __forceinline__ void fused_tile(const float* __restrict__ a, P n, con
 #pragma unroll
         for (uint32_t i = 0; i < kMaxPer; ++i) {
             const uint32_t e = tid + kFusedThreads * i;
-            res[i] = VP{f_inf(), kNone};
+            res[i] = VP{f_inf(), kNoPos};
             if (e < cnt) {
                 for (uint32_t j = 0; j < fan; ++j) vp_take(res[i], sv[e * fan + j], sp[e * fan + j]);
             }
@@ -158,19 +149,9 @@ struct TailPlan {
     uint64_t coff[kMaxLevels];  // first counter of level k, depth < k <= top
 };
 
-template <typename P>
-__device__ __forceinline__ P ldcg_pos(const P* p);
-template <>
-__device__ __forceinline__ uint32_t ldcg_pos(const uint32_t* p) { return __ldcg(p); }
-template <>
-__device__ __forceinline__ uint64_t ldcg_pos(const uint64_t* p) {
-    return __ldcg(reinterpret_cast<const unsigned long long*>(p));
-}
-
-template <int R, typename P>
-__device__ __forceinline__ void tail_upward(const LevelOutT<P>& out, const TailPlan& tp, uint64_t tile) {
+template <int R>
+__device__ __forceinline__ void tail_upward(const LevelOut& out, const TailPlan& tp, uint64_t tile) {
     constexpr uint32_t RF = 1u << R;
-    constexpr P kNone = IdxTraits<P>::none;
     __shared__ unsigned s_go;
     __threadfence();  // this tile's level entries before its arrival
     __syncthreads();
@@ -192,16 +173,16 @@ __device__ __forceinline__ void tail_upward(const LevelOutT<P>& out, const TailP
         __threadfence();  // the children's writers fenced before arriving
         const uint64_t child = (g << R) + lane;
         float v = f_inf();
-        P p = kNone;
+        uint32_t p = kNoPos;
         if (lane < RF && child < uint64_t(out.size[k - 1])) {
             v = __ldcg(out.val[k - 1] + child);
-            p = out.idx[k - 1] != nullptr ? ldcg_pos(out.idx[k - 1] + child) : P(child);
+            p = out.idx[k - 1] != nullptr ? __ldcg(out.idx[k - 1] + child) : uint32_t(child);
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             const float ov = __shfl_xor_sync(0xffffffffu, v, o);
-            const P op = __shfl_xor_sync(0xffffffffu, p, o);
-            if (op != kNone && (p == kNone || ov < v || (ov == v && op < p))) {
+            const uint32_t op = __shfl_xor_sync(0xffffffffu, p, o);
+            if (op != kNoPos && (p == kNoPos || ov < v || (ov == v && op < p))) {
                 v = ov;
                 p = op;
             }
@@ -228,17 +209,17 @@ __device__ __forceinline__ void tail_upward(const LevelOutT<P>& out, const TailP
 // Single CTA: builds levels from+1 .. last from level `from` (already built),
 // level after level, with a block barrier between levels (global writes of
 // the block are visible to it after __syncthreads).
-template <int R, typename P>
-__device__ __forceinline__ void tail_levels(const LevelOutT<P>& out, uint32_t from, uint32_t last) {
+template <int R>
+__device__ __forceinline__ void tail_levels(const LevelOut& out, uint32_t from, uint32_t last) {
     constexpr uint32_t RF = 1u << R;
     for (uint32_t k = from; k < last; ++k) {
         const float* src = out.val[k];
-        const P* src_idx = out.idx[k];
-        const P src_size = out.size[k];
-        for (P e = threadIdx.x; e < out.size[k + 1]; e += blockDim.x) {
-            VPT<P> c{f_inf(), IdxTraits<P>::none};
+        const uint32_t* src_idx = out.idx[k];
+        const uint32_t src_size = out.size[k];
+        for (uint32_t e = threadIdx.x; e < out.size[k + 1]; e += blockDim.x) {
+            VP c{f_inf(), kNoPos};
             for (uint32_t j = 0; j < RF; ++j) {
-                const P ch = e * RF + j;
+                const uint32_t ch = e * RF + j;
                 if (ch < src_size) vp_take(c, src[ch], src_idx != nullptr ? src_idx[ch] : ch);
             }
             out.val[k + 1][e] = c.v;

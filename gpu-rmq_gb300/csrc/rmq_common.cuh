@@ -57,16 +57,6 @@ struct Layout {
     uint64_t total = 0;                // entries in the level buffer incl. alignment padding
 };
 
-// Descriptor of one array inside packed buffers (batched and served modes).
-struct ArrayDesc {
-    uint64_t val_off;   // first value of the array, in floats from the values base
-    uint64_t lvl_base;  // first entry of its coarse levels, from the level-value base
-    uint64_t idx_base;  // first entry of its argmin arrays, from the argmin base
-    uint32_t num_levels;
-    uint32_t size[kMaxLevels];
-    uint32_t off[kMaxLevels];  // level k >= 1 starts at lvl_base + off[k]
-};
-
 // Index width: 32-bit handles (the reference's default nType = uint32_t,
 // uint2 queries) or 64-bit handles (its IS_LONG build: uint64_t, ulong2
 // queries; src/main.cu:21-27).
@@ -87,15 +77,12 @@ struct IdxTraits<uint64_t> {
 
 // Device-side view passed by value to the kernels (fits easily in the 32 KB
 // parameter space).
-template <typename I>
-struct LevelsT {
+struct Levels {
     const float* val[kMaxLevels];  // val[0] = caller's array
-    const I* idx[kMaxLevels];      // idx[k] (k >= 1): level-0 index of block k's first minimum
-    I size[kMaxLevels];
+    const uint32_t* idx[kMaxLevels];  // idx[k] (k >= 1): level-0 index of block k's first minimum
+    uint32_t size[kMaxLevels];
     uint32_t num_levels;
 };
-using Levels = LevelsT<uint32_t>;
-using Levels64 = LevelsT<uint64_t>;
 
 // ---------------------------------------------------------------------------
 // Memory access helpers (inline PTX; sm_100+ 256-bit global loads).  The
@@ -122,43 +109,10 @@ __device__ __forceinline__ void ld_sector_policy(const float* p, float (&v)[8], 
         : "l"(p), "l"(pol));
 }
 
-// Eight consecutive uint32 (one 32-byte sector) with an L2 cache policy.
-// The same load, allocating in L1 (for the small top levels, which every SM
-// re-reads for many queries).
-__device__ __forceinline__ void ld_sector_l1_policy(const float* p, float (&v)[8], uint64_t pol) {
-    asm(
-        "ld.global.nc.L2::cache_hint.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8], %9;"
-        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]),
-          "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
-        : "l"(p), "l"(pol));
-}
-
-__device__ __forceinline__ void ld_sector_u32_l1_policy(const uint32_t* p, uint32_t (&v)[8], uint64_t pol) {
-    asm(
-        "ld.global.nc.L2::cache_hint.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8], %9;"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]),
-          "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-        : "l"(p), "l"(pol));
-}
-
-__device__ __forceinline__ void ld_sector_u32_policy(const uint32_t* p, uint32_t (&v)[8], uint64_t pol) {
-    asm(
-        "ld.global.nc.L1::no_allocate.L2::cache_hint.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8], %9;"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]),
-          "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-        : "l"(p), "l"(pol));
-}
-
 __device__ __forceinline__ float fmin3(float a, float b, float c) {
     float d;
     asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
     return d;
-}
-
-__device__ __forceinline__ void ld_quad(const float* p, float (&v)[4]) {
-    asm("ld.global.nc.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];"
-                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
-                 : "l"(p));
 }
 
 __device__ __forceinline__ uint64_t policy_evict_last() {
@@ -223,37 +177,6 @@ __device__ __forceinline__ void st_stream(uint32_t* p, uint32_t v) {
 #else
     *p = v;
 #endif
-}
-
-// ---------------------------------------------------------------------------
-// Candidate ordering.  A candidate is an entry of some level together with the
-// level-0 position of its block start.  The pieces a query visits partition
-// [l, r], so positions are unique and ordering candidates by (value, position)
-// with IEEE "<" on the value reproduces the brute-force scan's
-// "first occurrence of the minimum" (src/cpu_methods.h:42-53).
-// ---------------------------------------------------------------------------
-struct Cand {
-    float v;
-    uint32_t pos;   // level-0 position of the candidate's block start
-    uint32_t lvl;   // level the candidate came from
-};
-
-__device__ __forceinline__ void cand_init(Cand& c) {
-    c.v = __int_as_float(0x7f800000);  // +inf
-    c.pos = kNoPos;
-    c.lvl = 0;
-}
-
-__device__ __forceinline__ bool cand_better(float v, uint32_t pos, const Cand& c) {
-    return (v < c.v) | ((v == c.v) & (pos < c.pos));
-}
-
-__device__ __forceinline__ void cand_update(Cand& c, float v, uint32_t pos, uint32_t lvl) {
-    if (cand_better(v, pos, c)) {
-        c.v = v;
-        c.pos = pos;
-        c.lvl = lvl;
-    }
 }
 
 __device__ __forceinline__ float f_inf() { return __int_as_float(0x7f800000); }

@@ -7,6 +7,7 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include "rmq_common.cuh"
+#include "rmq_window.cuh"
 
 namespace rmq {
 
@@ -30,11 +31,14 @@ Layout plan_layout(uint64_t n, uint64_t t, uint32_t rf_log);
 // the fused kernel (one launch in all); without, by extra launches.
 cudaError_t launch_build(const Layout& lay, const float* d_values, float* val_buf,
                          uint32_t* idx_buf, cudaStream_t s, unsigned* counters = nullptr);
-// Same with 64-bit positions (arrays beyond 2^32 entries).
-cudaError_t launch_build64(const Layout& lay, const float* d_values, float* val_buf,
-                           uint64_t* idx_buf, cudaStream_t s, unsigned* counters = nullptr);
 // Arrival counters the single-launch build needs for `lay` (0: none).
 uint64_t tail_counters(const Layout& lay);
+
+// Window tables (rmq_window.cuh) of n values into `tables` (window_bytes
+// bytes, 32-byte aligned).
+uint64_t window_bytes(uint64_t n, bool with_index);
+cudaError_t launch_window_build(const float* d_values, void* tables, uint64_t n, bool with_index, bool wide,
+                                cudaStream_t s);
 
 struct QueryArgs {
     Levels lv;
@@ -42,8 +46,10 @@ struct QueryArgs {
     uint64_t q;
     float* out_min;      // may be null for argmin queries
     uint32_t* out_idx;   // null for min queries
-    bool wide;           // 64-bit positions: lv64 / qs64 / out_idx64 are used instead
-    Levels64 lv64;
+    WinView win;         // VL: the window tables (lv is CL's)
+    bool host_buffers;   // queries and results in host memory, over the CPU-GPU link
+    bool wide;           // 64-bit positions: win64 / qs64 / out_idx64 are used instead
+    WinView64 win64;
     const uint64_t* qs64;
     uint64_t* out_idx64;
     uint32_t* err;       // invalid-query counter or null
@@ -56,13 +62,20 @@ struct QueryArgs {
 };
 
 cudaError_t launch_query(const QueryArgs& a, cudaStream_t s);
+// The window-table queries of launch_query (variants VL and VL_SHORT).
+cudaError_t launch_window_query(const QueryArgs& a, cudaStream_t s);
 
 cudaError_t launch_bruteforce(const float* vals, uint32_t n, const uint2* qs, uint32_t q,
                               float* out_min, uint32_t* out_idx, cudaStream_t s);
 
+// Queries per work unit: threads x kBatchLaneQueries of a batched CTA, and of
+// a warp of the served kernel.
+constexpr uint32_t kBatchLaneQueries = 4;
+constexpr uint32_t kServeUnit = 32;
+
 // Query launch over packed work: entry e (an array, or a request's array in
-// serving mode) owns queries [q_off[e], q_off[e+1]) of qs, in units of 32
-// queries per warp; owner[u] gives the entry of unit u (launch_fill_owner).
+// serving mode) owns queries [q_off[e], q_off[e+1]) of qs, in units of
+// threads x kBatchLaneQueries; owner[u] gives the entry of unit u (launch_fill_owner).
 struct BatchQueryArgs {
     const float* values;
     const ArrayDesc* descs;
@@ -70,8 +83,7 @@ struct BatchQueryArgs {
     const uint64_t* unit_off;
     const uint64_t* q_off;
     uint64_t total_units;
-    const float* lvl_val;
-    const uint32_t* lvl_idx;
+    const char* tables;
     const uint2* qs;
     float* out_min;
     uint32_t* out_idx;  // null: minima only
@@ -92,7 +104,7 @@ struct ServeIO {
 
 // The served batch: entry e (a request) answers its q_off[e+1] - q_off[e]
 // queries through io[e] and counts its invalid queries in bad[e] (zeroed by
-// the caller); units of 32 queries as for launch_batch_query.
+// the caller); units of kServeUnit queries.
 struct ServeQueryArgs {
     const float* values;
     const ArrayDesc* descs;
@@ -100,8 +112,7 @@ struct ServeQueryArgs {
     const uint64_t* unit_off;
     const uint64_t* q_off;
     uint64_t total_units;
-    const float* lvl_val;
-    const uint32_t* lvl_idx;
+    const char* tables;
     const ServeIO* io;
     uint32_t* bad;
     uint32_t threads;  // CTA size, multiple of 32, <= 512
@@ -110,10 +121,37 @@ struct ServeQueryArgs {
 cudaError_t launch_serve_query(const ServeQueryArgs& a, cudaStream_t s);
 cudaError_t launch_fill_owner(const uint64_t* unit_off, uint32_t num, uint32_t* owner, cudaStream_t s);
 
+// Kernel launch with the handle's L2 access-policy window, when it has one.
+template <typename K, typename... Args>
+static cudaError_t launch_with_window(K kernel, uint32_t grid, uint32_t block, const QueryArgs& a,
+                                      cudaStream_t s, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = 0;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    if (a.persist_base != nullptr && a.persist_bytes > 0) {
+        attr[0].id = cudaLaunchAttributeAccessPolicyWindow;
+        attr[0].val.accessPolicyWindow.base_ptr = const_cast<void*>(a.persist_base);
+        attr[0].val.accessPolicyWindow.num_bytes = a.persist_bytes;
+        attr[0].val.accessPolicyWindow.hitRatio = a.persist_hit_ratio;
+        attr[0].val.accessPolicyWindow.hitProp = cudaAccessPropertyPersisting;
+        attr[0].val.accessPolicyWindow.missProp = cudaAccessPropertyStreaming;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    } else {
+        cfg.attrs = nullptr;
+        cfg.numAttrs = 0;
+    }
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 #if RMQ_DEBUG_BOUNDS
 // Violations counted by the checked kernels of the query / batched units
 // since the last read (each read clears them).
 unsigned int bounds_bad_query();
+unsigned int bounds_bad_window();
 unsigned int bounds_bad_batch();
 #endif
 

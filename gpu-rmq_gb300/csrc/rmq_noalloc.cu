@@ -5,7 +5,7 @@
 // pool (a further cudaMalloc fails or fragments that pool), and latency-bound
 // callers for whom cudaMalloc / cudaFree are off limits because those calls
 // can block and synchronise the device.  For them this file keeps the
-// hierarchy's coarse levels in one file-scope device array of fixed size.
+// window tables in one file-scope device array of fixed size.
 // The caller still provides the values, the queries and the output buffers.
 //
 // When the array exists on a device: CUDA loads device code lazily by default
@@ -27,12 +27,11 @@
 
 namespace {
 
-// 8 MiB: coarse levels (fp32 value + uint32 index per entry) of arrays of up
-// to 2^22 entries at rf = 8 take about 4.8 MiB.
+// 8 MiB: the window tables of arrays of up to 2^22 entries take 4.3 MiB.
 constexpr size_t kScratchBytes = size_t(8) << 20;
 constexpr uint64_t kStaticMaxN = uint64_t(1) << 22;
 constexpr uint32_t kStaticRfLog = 3;
-constexpr uint64_t kStaticDefaultT = 32;
+constexpr uint64_t kStaticDefaultT = 32;  // checked as rmq_build checks it; the tables do not depend on it
 constexpr int kMaxDevices = 64;
 
 // Shared by every call on a device; it keeps the last call's contents.
@@ -117,35 +116,26 @@ extern "C" int rmq_query_idx_static(const float* d_values, uint64_t n, uint64_t 
     if (n > kStaticMaxN || q > 0xFFFFFFFFull) return RMQ_ERR_UNSUPPORTED;  // above the fixed scratch
     const uint64_t t = scan_threshold != 0 ? scan_threshold : kStaticDefaultT;
     if (t < (uint64_t(1) << kStaticRfLog)) return RMQ_ERR_ARG;  // VL precondition, src/xxx.h:938
-    const rmq::Layout lay = rmq::plan_layout(n, t, kStaticRfLog);
-    if (lay.total * (sizeof(float) + sizeof(uint32_t)) > kScratchBytes) return RMQ_ERR_UNSUPPORTED;
+    if (rmq::window_bytes(n, true) > kScratchBytes) return RMQ_ERR_UNSUPPORTED;
 
     void* scratch = nullptr;
     const int st = scratch_for_current_device(&scratch);
     if (st != RMQ_OK) return st;
-    float* val_buf = static_cast<float*>(scratch);
-    uint32_t* idx_buf = reinterpret_cast<uint32_t*>(val_buf + lay.total);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
 
-    // Every level entry a query reads is rewritten by the build of this call, so nothing
+    // Every table entry a query reads is rewritten by the build of this call, so nothing
     // in the scratch needs clearing between calls.
-    cudaError_t e = rmq::launch_build(lay, d_values, val_buf, idx_buf, s);
+    cudaError_t e = rmq::launch_window_build(d_values, scratch, n, true, false, s);
     if (e == cudaSuccess && q > 0) {
         rmq::QueryArgs a;
         std::memset(&a, 0, sizeof(a));
-        for (uint32_t k = 0; k < lay.num_levels; ++k) {
-            a.lv.val[k] = k == 0 ? d_values : val_buf + lay.offset[k];
-            a.lv.idx[k] = k == 0 ? nullptr : idx_buf + lay.offset[k];
-            a.lv.size[k] = uint32_t(lay.size[k]);
-        }
-        a.lv.num_levels = lay.num_levels;
+        a.win = rmq::win_view<uint32_t>(d_values, scratch, n, true);
         a.qs = reinterpret_cast<const uint2*>(d_lr);
         a.q = q;
         a.out_min = d_min_or_null;
         a.out_idx = d_argmin;
         a.variant = RMQ_VARIANT_VL;
-        a.lanes = 8;
-        a.rf_log = lay.rf_log;
+        a.rf_log = kStaticRfLog;
         e = rmq::launch_query(a, s);
     }
     if (e != cudaSuccess) {

@@ -8,28 +8,14 @@
 // partition [l, r], so the minimum is the minimum over the pieces and the
 // argmin is the lowest-position candidate among those equal to it.
 //
-// Two work distributions share that descent:
-//   VL  one thread per query, 256-bit sector loads (reference alg 20,
-//       kernel_hierarchical_vector_load, src/xxx.h:883-930, which uses float4);
-//   CL  a tile of G lanes answers its G queries one after another, the lanes
-//       sharing each query's sectors (reference alg 16, xxx_query,
-//       src/xxx.h:124-200).
+// CL walks it: a tile of G lanes answers its G queries one after another, the
+// lanes sharing each query's sectors (reference alg 16, xxx_query,
+// src/xxx.h:124-200).  VL (reference alg 20, kernel_hierarchical_vector_load,
+// src/xxx.h:883-930) has its own tables and kernels (rmq_window.cuh).
 #include "rmq_internal.h"
-#include "rmq_vl.cuh"
+#include "rmq_cl.cuh"
 
 namespace rmq {
-
-// CAP: the short-query variant (RMQ_VARIANT_VL_SHORT), which takes a short
-// query's level-0 winner in phase 1 instead of reading it again in phase 2.
-template <int R, bool ARGMIN, typename I, bool CAP = false>
-__global__ void __launch_bounds__(256)
-query_vl_kernel(LevelsT<I> lv, const typename IdxTraits<I>::Pair* __restrict__ qs, uint64_t q,
-                float* __restrict__ out_min, I* __restrict__ out_idx, uint32_t* __restrict__ err) {
-    // No early return: every lane takes part in the warp's long final scans.
-    using C = typename IdxTraits<I>::Count;
-    const C i = C(blockIdx.x) * blockDim.x + threadIdx.x;
-    vl_answer<R, ARGMIN, I, CAP>(lv, qs, i, i < q, out_min, out_idx, err);
-}
 
 // ---------------------------------------------------------------------------
 // CL: a tile of G lanes per query, queries of the tile one after another
@@ -63,7 +49,7 @@ __device__ __forceinline__ void cl_sector(const Levels& lv, uint32_t k, uint32_t
     const uint32_t jlo = s < lo ? lo - s : 0u;
     const uint32_t jhi = hi - s < 8u ? hi - s : 8u;
     float v[8];
-    load_level_sector<uint32_t, false>(lv, k, s, pol, v);
+    load_level_sector(lv, k, s, pol, v);
     const float sm = sector_min(v, jlo, jhi);
     if (ARGMIN) {
         if (sm < b.v || (sm == b.v && key < b.key)) {
@@ -138,7 +124,7 @@ __device__ __forceinline__ void cl_locate(const Levels& lv, const LaneBest& b, f
     const uint32_t jlo = (b.meta >> 8) & 0xffu;
     const uint32_t jhi = (b.meta >> 16) & 0xffu;
     float v[8];
-    load_level_sector<uint32_t, false>(lv, k, b.s, pol, v);
+    load_level_sector(lv, k, b.s, pol, v);
     uint32_t jj = jlo;
 #pragma unroll
     for (int t = 7; t >= 0; --t)
@@ -344,39 +330,9 @@ bruteforce_kernel(const float* __restrict__ a, uint32_t n, const uint2* __restri
 // Launchers
 // ---------------------------------------------------------------------------
 
-template <typename K, typename... Args>
-static cudaError_t launch_with_window(K kernel, uint32_t grid, uint32_t block, const QueryArgs& a,
-                                      cudaStream_t s, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    if (a.persist_base != nullptr && a.persist_bytes > 0) {
-        attr[0].id = cudaLaunchAttributeAccessPolicyWindow;
-        attr[0].val.accessPolicyWindow.base_ptr = const_cast<void*>(a.persist_base);
-        attr[0].val.accessPolicyWindow.num_bytes = a.persist_bytes;
-        attr[0].val.accessPolicyWindow.hitRatio = a.persist_hit_ratio;
-        attr[0].val.accessPolicyWindow.hitProp = cudaAccessPropertyPersisting;
-        attr[0].val.accessPolicyWindow.missProp = cudaAccessPropertyStreaming;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-    } else {
-        cfg.attrs = nullptr;
-        cfg.numAttrs = 0;
-    }
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
-// Query kernels run in 128-thread blocks.  A block keeps its register slots
-// until its last query ends, so smaller blocks give finished warps' slots
-// back sooner; at the same registers per thread the SM holds as many warps
-// (VL 32-bit: 12 blocks of 128 = 6 of 256).  n = q = 2^26, lognormal
-// lengths, vs 256-thread blocks: VL +0.5 % (three-way mixture +1.7 %,
-// uniform lengths -0.5 %), VL with 64-bit positions +6.3 % (55 registers:
-// 9 blocks of 128 hold 36 warps, 4 of 256 held 32), CL (rf 8, 2 lanes)
-// +2.1 %.  64-thread blocks: within 1 % of these, uniform lengths -1 %.
+// 128-thread blocks: a block keeps its register slots until its last query
+// ends, so smaller blocks give finished warps' slots back sooner (CL, rf 8,
+// 2 lanes, n = q = 2^26, lognormal lengths: +2.1 % over 256).
 constexpr uint32_t kQueryBlock = 128;
 
 template <int R, int MODE>
@@ -399,29 +355,8 @@ static cudaError_t launch_cl(const QueryArgs& a, cudaStream_t s, uint32_t grid, 
 
 template <int R>
 static cudaError_t launch_query_r(const QueryArgs& a, cudaStream_t s) {
-    const bool argmin = a.out_idx != nullptr || a.out_idx64 != nullptr;
+    const bool argmin = a.out_idx != nullptr;
     const uint32_t grid = uint32_t((a.q + kQueryBlock - 1u) / kQueryBlock);
-    if (a.wide) {
-        // 64-bit positions: the VL kernel only (the short-query variant is VL here).
-        if (a.variant != 2 && a.variant != 6) return cudaErrorNotSupported;
-        const ulonglong2* qs = reinterpret_cast<const ulonglong2*>(a.qs64);
-        return argmin ? launch_with_window(query_vl_kernel<R, true, uint64_t>, grid, kQueryBlock, a, s, a.lv64,
-                                             qs, a.q, a.out_min, a.out_idx64, a.err)
-                      : launch_with_window(query_vl_kernel<R, false, uint64_t>, grid, kQueryBlock, a, s, a.lv64,
-                                             qs, a.q, a.out_min, static_cast<uint64_t*>(nullptr), a.err);
-    }
-    if (a.variant == 6 && R == 3) {
-        return argmin ? launch_with_window(query_vl_kernel<3, true, uint32_t, true>, grid, kQueryBlock, a, s, a.lv,
-                                           a.qs, a.q, a.out_min, a.out_idx, a.err)
-                      : launch_with_window(query_vl_kernel<3, false, uint32_t, true>, grid, kQueryBlock, a, s, a.lv,
-                                           a.qs, a.q, a.out_min, static_cast<uint32_t*>(nullptr), a.err);
-    }
-    if (a.variant == 2 || a.variant == 6) {
-        return argmin ? launch_with_window(query_vl_kernel<R, true, uint32_t>, grid, kQueryBlock, a, s, a.lv,
-                                             a.qs, a.q, a.out_min, a.out_idx, a.err)
-                      : launch_with_window(query_vl_kernel<R, false, uint32_t>, grid, kQueryBlock, a, s, a.lv,
-                                             a.qs, a.q, a.out_min, static_cast<uint32_t*>(nullptr), a.err);
-    }
     const uint32_t q32 = uint32_t(a.q);
     switch (a.variant) {
         case 1: return launch_cl<R, kClShuffle>(a, s, grid, q32, argmin);
@@ -444,6 +379,7 @@ RMQ_BOUNDS_COUNTER_READER(bounds_bad_query)
 
 cudaError_t launch_query(const QueryArgs& a, cudaStream_t s) {
     if (a.q == 0) return cudaSuccess;
+    if (a.variant == 2 || a.variant == 6) return launch_window_query(a, s);
     switch (a.rf_log) {
         case 3: return launch_query_r<3>(a, s);
         case 4: return launch_query_r<4>(a, s);

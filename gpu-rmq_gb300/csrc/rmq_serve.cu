@@ -50,8 +50,7 @@ using rmq::Arena;
 struct ServedArray {
     uint64_t n = 0, seed = 0;
     const float* host = nullptr;
-    rmq::Layout lay;
-    uint64_t bytes = 0, val_bytes = 0, lvl_bytes = 0;
+    uint64_t bytes = 0, val_bytes = 0;
     bool resident = false, ready = false, admitted_before = false;
     uint64_t off = 0;  // arena byte offset
     int pins = 0;
@@ -152,17 +151,7 @@ struct rmq_server {
 namespace {
 
 rmq::ArrayDesc describe(const ServedArray& a) {
-    rmq::ArrayDesc d;
-    std::memset(&d, 0, sizeof(d));
-    d.val_off = a.off / 4;
-    d.lvl_base = (a.off + a.val_bytes) / 4;
-    d.idx_base = (a.off + a.val_bytes + a.lvl_bytes) / 4;
-    d.num_levels = a.lay.num_levels;
-    for (uint32_t k = 0; k < a.lay.num_levels; ++k) {
-        d.size[k] = uint32_t(a.lay.size[k]);
-        d.off[k] = k == 0 ? 0u : uint32_t(a.lay.offset[k]);
-    }
-    return d;
+    return rmq::win_desc(a.off / 4, a.off + a.val_bytes, rmq::win_shape(a.n, true));
 }
 
 void evict(rmq_server* s, uint64_t id) {
@@ -190,8 +179,6 @@ bool admit(rmq_server* s, uint64_t id) {
     a.ready = false;
     a.last_use = ++s->use_clock;
     float* vals = reinterpret_cast<float*>(s->arena + a.off);
-    float* lvl = reinterpret_cast<float*>(s->arena + a.off + a.val_bytes);
-    uint32_t* idx = reinterpret_cast<uint32_t*>(s->arena + a.off + a.val_bytes + a.lvl_bytes);
     int st = RMQ_OK;
     if (a.host != nullptr) {
         st = cudaMemcpyAsync(vals, a.host, a.n * sizeof(float), cudaMemcpyHostToDevice, s->build_stream) ==
@@ -199,7 +186,7 @@ bool admit(rmq_server* s, uint64_t id) {
     } else {
         st = rmq_gen_values_device(vals, a.n, a.seed, reinterpret_cast<rmq_stream_t>(s->build_stream));
     }
-    if (st == RMQ_OK && rmq::launch_build(a.lay, vals, lvl, idx, s->build_stream) != cudaSuccess) st = RMQ_ERR_CUDA;
+    if (st == RMQ_OK && rmq::launch_window_build(vals, s->arena + a.off + a.val_bytes, a.n, true, false, s->build_stream) != cudaSuccess) st = RMQ_ERR_CUDA;
     if (st == RMQ_OK && cudaEventRecord(a.built, s->build_stream) != cudaSuccess) st = RMQ_ERR_CUDA;
     if (st != RMQ_OK) {
         cudaGetLastError();
@@ -316,7 +303,7 @@ bool launch_batch(rmq_server* s, Slot& sl, std::unique_lock<std::mutex>& lk) {
     hu[0] = 0;
     for (uint32_t i = 0; i < nr; ++i) {
         hq[i + 1] = hq[i] + reqs[i]->q;
-        hu[i + 1] = hu[i] + (reqs[i]->q + 31) / 32;
+        hu[i + 1] = hu[i] + (reqs[i]->q + rmq::kServeUnit - 1) / rmq::kServeUnit;
     }
     uint32_t* h_owner = reinterpret_cast<uint32_t*>(sl.h_in + hdr);
     const size_t qat = hdr + owner_bytes(hu[nr]);
@@ -364,8 +351,7 @@ bool launch_batch(rmq_server* s, Slot& sl, std::unique_lock<std::mutex>& lk) {
         a.unit_off = du;
         a.q_off = dq;
         a.total_units = hu[nr];
-        a.lvl_val = reinterpret_cast<const float*>(s->arena);
-        a.lvl_idx = reinterpret_cast<const uint32_t*>(s->arena);
+        a.tables = reinterpret_cast<const char*>(s->arena);
         a.io = reinterpret_cast<const rmq::ServeIO*>(du + (nr + 1));
         a.bad = reinterpret_cast<uint32_t*>(sl.d_out);
         a.threads = s->cfg.query_threads;
@@ -452,11 +438,8 @@ int register_array(rmq_server* s, uint64_t n, uint64_t seed, const float* host, 
     a.n = n;
     a.seed = seed;
     a.host = host;
-    a.lay = rmq::plan_layout(n, s->cfg.scan_threshold, 3);
     a.val_bytes = rmq::arena_round_up(n * sizeof(float));
-    const uint64_t lvl_entries = a.lay.num_levels > 1 ? a.lay.total : 0;
-    a.lvl_bytes = rmq::arena_round_up(lvl_entries * sizeof(float));
-    a.bytes = a.val_bytes + 2 * a.lvl_bytes;
+    a.bytes = a.val_bytes + rmq::arena_round_up(rmq::window_bytes(n, true));
     if (a.bytes > s->cfg.hbm_budget_bytes) return RMQ_ERR_OOM;
     if (cudaEventCreateWithFlags(&a.built, cudaEventDisableTiming) != cudaSuccess) return RMQ_ERR_CUDA;
     std::lock_guard<std::mutex> lock(s->mu);
@@ -512,7 +495,7 @@ int rmq_server_create(const rmq_server_config* cfg_in, rmq_server** out) {
     for (Slot& sl : s->slots) {
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&sl.stream, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming);
-        const size_t in_bytes = header_bytes(mr) + owner_bytes(mq / 32 + mr) + mq * 2 * sizeof(uint32_t);
+        const size_t in_bytes = header_bytes(mr) + owner_bytes(mq / rmq::kServeUnit + mr) + mq * 2 * sizeof(uint32_t);
         const size_t out_bytes = bad_bytes(mr) + mq * 8;
         if (e == cudaSuccess) e = cudaMallocHost(&sl.h_in, in_bytes);
         if (e == cudaSuccess) e = cudaMallocHost(&sl.h_out, out_bytes);

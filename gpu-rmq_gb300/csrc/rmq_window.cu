@@ -1,0 +1,177 @@
+// rmq_window.cu — the single-array kernels of the window tables: build
+// (rmq_window_build.cuh) and queries (rmq_window.cuh).
+//
+// The build kernels after the first are launched with programmatic stream
+// serialization, so each is scheduled before its predecessor ends and no
+// launch gap separates them.
+#include "rmq_internal.h"
+#include "rmq_window_build.cuh"
+
+namespace rmq {
+
+__device__ __forceinline__ void wait_previous_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void allow_next_grid() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+__global__ void __launch_bounds__(kBlockThreads) win_block_kernel(WinOut w) {
+    allow_next_grid();
+    win_block_tile(w, blockIdx.x);
+}
+
+__global__ void __launch_bounds__(256) win_low_kernel(WinOut w) {
+    __shared__ uint2 sa[kSpan + kHaloLow], sb[kSpan + kHaloLow];
+    wait_previous_grid();
+    allow_next_grid();
+    win_low_tile(w, blockIdx.x, sa, sb);
+}
+
+__global__ void __launch_bounds__(256) win_mid_kernel(WinOut w) {
+    __shared__ uint2 sa[kSpan + kHaloMid], sb[(kSpan + kHaloMid) / 2];
+    wait_previous_grid();
+    allow_next_grid();
+    win_mid_tile(w, blockIdx.x, sa, sb);
+}
+
+__global__ void __launch_bounds__(1024) win_top_kernel(WinOut w) {
+    wait_previous_grid();
+    win_top(w);
+}
+
+// Launch with programmatic stream serialization (the kernel waits for its
+// predecessor in wait_previous_grid).
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_dependent(void (*kernel)(KArgs...), uint32_t grid, uint32_t block, cudaStream_t s,
+                                    Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+cudaError_t launch_window_build(const float* d_values, void* tables, uint64_t n, bool with_index, bool wide,
+                                cudaStream_t s) {
+    const WinShape sh = win_shape(n, with_index);
+    WinOut w;
+    char* b = static_cast<char*>(tables);
+    w.a = d_values;
+    w.v1 = reinterpret_cast<float*>(b);
+    w.j1 = reinterpret_cast<uint8_t*>(b + sh.j1_off);
+    w.t = reinterpret_cast<uint2*>(b + sh.t_off);
+    w.n = n;
+    w.S = sh.S;
+    w.cb = sh.cb;
+    w.blk = sh.blk;
+    w.gb = sh.gb;
+    w.c = sh.c;
+    w.first = sh.first;
+    w.kmax = sh.kmax;
+    w.wide = wide;
+    const WinTiles t = win_tiles(sh);
+    win_block_kernel<<<uint32_t(t.block), kBlockThreads, 0, s>>>(w);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess && t.low > 0) e = launch_dependent(win_low_kernel, uint32_t(t.low), 256, s, w);
+    if (e == cudaSuccess && t.mid > 0) e = launch_dependent(win_mid_kernel, uint32_t(t.mid), 256, s, w);
+    if (e == cudaSuccess && t.top > 0) e = launch_dependent(win_top_kernel, uint32_t(t.top), 1024, s, w);
+    return e;
+}
+
+uint64_t window_bytes(uint64_t n, bool with_index) {
+    return win_shape(n, with_index).bytes;
+}
+
+// ---------------------------------------------------------------------------
+// Queries.
+//
+// win_query_kernel (win_block: four queries per thread in a pass, the harder
+// ones listed in shared memory and answered by full warps) for launches that
+// fill the GPU, win_one_kernel (one query per thread, no lists, no barriers)
+// for the others.  n = 2^20, device time of one launch in us, the two kernels
+// and the block-minimum descent they replace:
+//
+//   queries                2^18               2^20                2^22
+//   uniform lengths     8.0  10.8  14.0   15.7  33.1  38.6    38.3  119  137
+//   lognormal(2^13, 1) 10.1  10.7  12.7   17.4  29.8  34.0    47.9  106  119
+//   lognormal(32, 0.7) 12.3   8.7   8.6   27.7  22.7  22.9    86.7   80   82
+//
+// The lengths are not known before the launch.  win_one_kernel answers up to
+// 2^18 queries, and up to 2^20 over a small array (blocks of eight entries),
+// where short queries are fast enough to notice the lists; at n = 2^26 the
+// lists win for every law from 2^19 on.  Results in host memory always come
+// from win_one_kernel: its warps write whole 128-byte lines, which the
+// CPU-GPU link wants (2^22 queries, page-locked: 214 us against 385).
+//
+// kQueryThreads and the blocks per SM: the loads in flight live in the part
+// of the SM's 256 KiB that shared memory leaves (8 KiB per block here); with
+// 16 KiB per block, or 32 KiB of shared memory more in all, the headline
+// workload (lognormal(2^13, 1), n = q = 2^26) takes 6 % to 100 % longer.
+constexpr uint32_t kQueryThreads = 128;
+constexpr uint32_t kLaneQueries = 4;
+constexpr uint32_t kBlockQueries = kQueryThreads * kLaneQueries;
+constexpr uint32_t kOneThreads = 64;
+constexpr uint64_t kFewQueries = uint64_t(1) << 18;
+constexpr uint64_t kFewQueriesSmall = uint64_t(1) << 20;
+
+template <bool ARGMIN, typename I>
+__global__ void __launch_bounds__(kQueryThreads, sizeof(I) == 4 ? 9 : 8)
+win_query_kernel(WinViewT<I> w, const typename IdxTraits<I>::Pair* __restrict__ qs, uint64_t q,
+                 float* __restrict__ out_min, I* __restrict__ out_idx, uint32_t* __restrict__ err) {
+    __shared__ __align__(16) unsigned char smem[win_lists_bytes<I>(kBlockQueries)];
+    const uint64_t at = uint64_t(blockIdx.x) * kBlockQueries;
+    const uint32_t cnt = q - at < kBlockQueries ? uint32_t(q - at) : kBlockQueries;
+    const WinLists<I> sm = win_lists<I>(smem, kBlockQueries);
+    const uint32_t bad = win_block<ARGMIN, kLaneQueries>(w, sm, kQueryThreads, qs + at, cnt,
+                                                         out_min != nullptr ? out_min + at : nullptr,
+                                                         ARGMIN ? out_idx + at : nullptr);
+    if (bad != 0u && err != nullptr) atomicAdd(err, bad);
+}
+
+template <bool ARGMIN, typename I>
+__global__ void __launch_bounds__(kOneThreads)
+win_one_kernel(WinViewT<I> w, const typename IdxTraits<I>::Pair* __restrict__ qs, uint64_t q,
+               float* __restrict__ out_min, I* __restrict__ out_idx, uint32_t* __restrict__ err) {
+    using C = typename IdxTraits<I>::Count;
+    const C i = C(blockIdx.x) * kOneThreads + threadIdx.x;
+    if (uint64_t(blockIdx.x) * kOneThreads + threadIdx.x >= q) return;
+    const typename IdxTraits<I>::Pair Q = ld_query(qs + i);
+    WinBest<I> c{f_nan(), IdxTraits<I>::none, false};
+    I l = IdxTraits<I>::none;
+    if (Q.x <= Q.y && Q.y < w.n) {
+        l = Q.x;
+        c = win_one(w, l, I(Q.y));
+    } else if (err != nullptr) {
+        atomicAdd(err, 1u);
+    }
+    if (out_min != nullptr) st_stream(out_min + i, c.v);
+    if (ARGMIN) st_stream(out_idx + i, win_place(w, c, l));
+}
+
+template <bool ARGMIN, typename I>
+static cudaError_t launch_window_typed(const QueryArgs& a, const WinViewT<I>& w,
+                                       const typename IdxTraits<I>::Pair* qs, I* out_idx, cudaStream_t s) {
+    if (a.q <= (w.n <= kSmallN ? kFewQueriesSmall : kFewQueries) || a.host_buffers)
+        return launch_with_window(win_one_kernel<ARGMIN, I>, uint32_t((a.q + kOneThreads - 1u) / kOneThreads), kOneThreads,
+                                  a, s, w, qs, a.q, a.out_min, out_idx, a.err);
+    return launch_with_window(win_query_kernel<ARGMIN, I>, uint32_t((a.q + kBlockQueries - 1u) / kBlockQueries),
+                              kQueryThreads, a, s, w, qs, a.q, a.out_min, out_idx, a.err);
+}
+
+cudaError_t launch_window_query(const QueryArgs& a, cudaStream_t s) {
+    if (a.wide) {
+        const ulonglong2* qs = reinterpret_cast<const ulonglong2*>(a.qs64);
+        return a.out_idx64 != nullptr ? launch_window_typed<true, uint64_t>(a, a.win64, qs, a.out_idx64, s)
+                                      : launch_window_typed<false, uint64_t>(a, a.win64, qs, nullptr, s);
+    }
+    return a.out_idx != nullptr ? launch_window_typed<true, uint32_t>(a, a.win, a.qs, a.out_idx, s)
+                                : launch_window_typed<false, uint32_t>(a, a.win, a.qs, nullptr, s);
+}
+
+#if RMQ_DEBUG_BOUNDS
+RMQ_BOUNDS_COUNTER_READER(bounds_bad_window)
+#endif
+
+}  // namespace rmq

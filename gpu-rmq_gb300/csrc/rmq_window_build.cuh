@@ -1,0 +1,230 @@
+// rmq_window_build.cuh — device functions of the window-table build, shared by
+// the single-array kernels (rmq_window.cu) and the batched ones (rmq_batch.cu).
+//
+// One streaming pass over level 0 writes the minimum and its offset for every
+// block of 16 entries (0.31 n bytes); everything above is computed from those,
+// which are still in L2.  A tile pass holds 2048 strides and a halo of 512 in
+// shared memory and makes every table whose windows fit the halo; a second
+// tile pass does the same for the next six sizes; one CTA makes the few
+// entries above.  Each table is one doubling of the one below:
+// T_(k+1)[i] = first minimum of T_k[2i] and T_k[2i + windows per stride].
+#pragma once
+
+#include "rmq_window.cuh"
+
+namespace rmq {
+
+constexpr uint32_t kBlockTile = 8192;      // level-0 entries per CTA of the block pass
+constexpr uint32_t kBlockThreads = 256;
+constexpr uint32_t kSpan = 2048;           // own strides per tile of the window kernels
+constexpr uint32_t kHaloLow = 512;         // halo of the first window kernel, in strides of 2^gb
+constexpr uint32_t kHaloMid = 1024;        // halo of the second, in its input's strides
+constexpr uint32_t kMidSteps = 6;          // sizes the second window kernel adds
+
+// Largest window the first kernel makes from a tile and its halo (512 strides
+// of 2^gb), and the second (its halo: 2^kMidSteps windows of that size).
+template <typename V>
+__host__ __device__ __forceinline__ uint32_t win_low_log(const V& w) { return w.gb + 9u; }
+template <typename V>
+__host__ __device__ __forceinline__ uint32_t win_mid_log(const V& w) { return w.gb + 9u + kMidSteps; }
+
+// Blocks of one tile.  A warp's load covers 32 consecutive sectors (1 KiB);
+// each lane takes its sector's first minimum, and the two lanes of a block
+// exchange one sector each of two loads, so that every lane ends with one
+// whole block and a warp stores 32 consecutive blocks.
+__device__ __forceinline__ void win_block_tile(const WinOut& w, uint64_t tile) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint64_t base = tile * kBlockTile;
+    const uint64_t sec0 = (base >> 3) + warp * 128u + lane;
+    const uint64_t pol = policy_evict_first();
+    float v[4][8];
+    if (base + kBlockTile <= w.n) {
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) ld_sector_policy(w.a + 8u * (sec0 + 32u * i), v[i], pol);
+    } else {
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) {
+            const uint64_t s = 8u * (sec0 + 32u * i);
+            if (s + 8u <= w.n) {
+                ld_sector_policy(w.a + s, v[i], pol);
+            } else {
+#pragma unroll
+                for (uint32_t j = 0; j < 8; ++j) v[i][j] = s + j < w.n ? w.a[s + j] : f_inf();
+            }
+        }
+    }
+    float m[4];
+    uint32_t off[4];
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i) {
+        const float x = fmin3(fmin3(v[i][0], v[i][1], v[i][2]), fmin3(v[i][3], v[i][4], v[i][5]),
+                              fminf(v[i][6], v[i][7]));
+        uint32_t j = 0;
+        float mv = v[i][0];  // the first equal entry's own bits (a zero keeps its sign)
+#pragma unroll
+        for (int jj = 7; jj >= 0; --jj) {
+            if (v[i][jj] == x) {
+                j = uint32_t(jj);
+                mv = v[i][jj];
+            }
+        }
+        m[i] = mv;
+        off[i] = j;
+    }
+    if (w.blk == 3u) {  // a sector is a block
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) {
+            const uint64_t blk = sec0 + 32u * i;
+            if ((blk << 3) < w.n) {
+                w.v1[blk] = m[i];
+                w.j1[blk] = uint8_t(off[i]);
+            }
+        }
+        return;
+    }
+    const bool odd = (lane & 1u) != 0u;
+#pragma unroll
+    for (uint32_t p = 0; p < 4; p += 2) {
+        const float mine = odd ? m[p + 1] : m[p];
+        const uint32_t mo = odd ? off[p + 1] : off[p];
+        const float other = __shfl_xor_sync(0xffffffffu, odd ? m[p] : m[p + 1], 1);
+        const uint32_t oo = __shfl_xor_sync(0xffffffffu, odd ? off[p] : off[p + 1], 1);
+        const float lov = odd ? other : mine, hiv = odd ? mine : other;
+        const uint32_t loo = odd ? oo : mo, hio = odd ? mo : oo;
+        const bool hi = hiv < lov;  // equal: the first sector's entry stays
+        const uint64_t blk = (sec0 + 32u * (odd ? p + 1u : p)) >> 1;
+        if ((blk << 4) < w.n) {
+            w.v1[blk] = hi ? hiv : lov;
+            w.j1[blk] = uint8_t(hi ? 8u + hio : loo);
+        }
+    }
+}
+
+// First minimum of two entries; hi_off: what the upper one's offset gains (0
+// for positions).
+__device__ __forceinline__ uint2 win_first(uint2 lo, uint2 hi, uint32_t hi_off) {
+    return __uint_as_float(hi.x) < __uint_as_float(lo.x) ? make_uint2(hi.x, hi.y + hi_off) : lo;
+}
+
+// Doubles T_k held in `src` (`cnt` entries from entry `at` of T_k) up to
+// T_(last), writing each table's own entries (the tile's kSpan strides of the
+// first source) to the table and keeping them in shared memory in turn.
+// Entries whose window starts at or past n do not exist and are never read.
+__device__ __forceinline__ void win_double_up(const WinOut& w, uint32_t k, uint32_t last, uint64_t at, uint32_t cnt,
+                                              uint32_t own, uint2* src, uint2* dst) {
+    const uint32_t wpu = 1u << w.c;
+    for (; k < last; ++k) {
+        const uint32_t s = win_stride_log(w, k + 1u);
+        const uint32_t half = 1u << k, off = w.wide ? half : 0u;  // k < 32
+        cnt >>= 1;
+        own >>= 1;
+        at >>= 1;
+        uint2* out = w.t + win_table_at<uint64_t>(w, k + 1u) + at;
+        for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) {
+            const uint64_t start = (at + i) << s;
+            if (start >= w.n) break;
+            uint2 e = src[2u * i];
+            const uint32_t h = 2u * i + wpu;
+            if (h < 2u * cnt && start + half < w.n) e = win_first(e, src[h], off);
+            dst[i] = e;
+            if (i < own) out[i] = e;
+        }
+        __syncthreads();
+        uint2* x = src;
+        src = dst;
+        dst = x;
+    }
+}
+
+// The tables up to T_(gb+9) (all of them when the array has one tile) of the
+// tile's kSpan strides of 2^gb entries.
+__device__ __forceinline__ void win_low_tile(const WinOut& w, uint64_t tile, uint2* sa, uint2* sb) {
+    const uint64_t g0 = tile * kSpan;
+    const uint32_t cnt = kSpan + kHaloLow;
+    const uint32_t bpg = 1u << (w.gb - w.blk);  // blocks per stride
+    const uint64_t nb = (w.n + (uint64_t(1) << w.blk) - 1) >> w.blk;
+    for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) {
+        if (g0 + i >= w.S) break;
+        const uint64_t b = (g0 + i) * bpg;
+        uint2 e = make_uint2(__float_as_uint(w.v1[b]), w.j1[b]);
+        for (uint32_t c = 1; c < bpg; ++c)
+            if (b + c < nb) e = win_first(e, make_uint2(__float_as_uint(w.v1[b + c]), w.j1[b + c]), c << w.blk);
+        if (!w.wide) e.y += uint32_t(b << w.blk);
+        sa[i] = e;
+    }
+    __syncthreads();
+    // Windows of 2, 4, 8 strides (2^first entries), the last one the first
+    // table; where the next one has the same stride, a doubling of 8.
+    uint2 *src = sa, *dst = sb;
+    const uint32_t kb = w.gb + w.c;
+    for (uint32_t d = 1; d <= (w.first < kb ? 8u : 4u); d <<= 1) {
+        uint2* out = nullptr;
+        if (d == 4u) out = w.t + win_table_at<uint64_t>(w, w.first) + g0;
+        if (d == 8u && w.kmax >= kb) out = w.t + win_table_at<uint64_t>(w, kb) + g0;
+        for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) {
+            if (g0 + i >= w.S) break;
+            uint2 e = src[i];
+            if (i + d < cnt && g0 + i + d < w.S) e = win_first(e, src[i + d], w.wide ? d << w.gb : 0u);
+            dst[i] = e;
+            if (out != nullptr && i < kSpan) out[i] = e;
+        }
+        __syncthreads();
+        uint2* x = src;
+        src = dst;
+        dst = x;
+    }
+    const uint32_t last = w.S <= kSpan ? w.kmax : (w.kmax < win_low_log(w) ? w.kmax : win_low_log(w));
+    win_double_up(w, kb, last, g0, cnt, kSpan, src, dst);
+}
+
+// The next kMidSteps tables above T_(gb+9) of one tile of its entries.
+__device__ __forceinline__ void win_mid_tile(const WinOut& w, uint64_t tile, uint2* sa, uint2* sb) {
+    const uint32_t k = win_low_log(w), s = win_stride_log(w, k);
+    const uint64_t e0 = tile * kSpan;
+    const uint32_t cnt = kSpan + kHaloMid;
+    const uint64_t entries = (w.n + (uint64_t(1) << s) - 1) >> s;
+    const uint2* src = w.t + win_table_at<uint64_t>(w, k) + e0;
+    for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) {
+        if (e0 + i >= entries) break;
+        sa[i] = __ldcg(src + i);
+    }
+    __syncthreads();
+    const uint32_t last = entries <= kSpan ? w.kmax : (w.kmax < win_mid_log(w) ? w.kmax : win_mid_log(w));
+    win_double_up(w, k, last, e0, cnt, kSpan, sa, sb);
+}
+
+// CTAs of each build kernel for one array (0: not needed).
+struct WinTiles {
+    uint64_t block, low, mid, top;
+};
+inline WinTiles win_tiles(const WinShape& w) {
+    WinTiles t{(w.n + kBlockTile - 1) / kBlockTile, 0, 0, 0};
+    if (w.t_entries == 0) return t;
+    t.low = (w.S + kSpan - 1) / kSpan;
+    if (t.low == 1 || w.kmax <= win_low_log(w)) return t;
+    const uint32_t s = win_stride_log(w, win_low_log(w));
+    t.mid = (((w.n + (uint64_t(1) << s) - 1) >> s) + kSpan - 1) / kSpan;
+    t.top = t.mid > 1 && w.kmax > win_mid_log(w) ? 1 : 0;
+    return t;
+}
+
+// The tables above T_(gb+15), by one CTA (at 2^26 entries: 512 entries and
+// halving), each from the one below in global memory.
+__device__ __forceinline__ void win_top(const WinOut& w) {
+    const uint32_t wpu = 1u << w.c;
+    for (uint32_t k = win_mid_log(w); k < w.kmax; ++k) {
+        const uint32_t s = win_stride_log(w, k + 1u);
+        const uint64_t entries = (w.n + (uint64_t(1) << s) - 1) >> s;
+        const uint2* src = w.t + win_table_at<uint64_t>(w, k);
+        uint2* dst = w.t + win_table_at<uint64_t>(w, k + 1u);
+        const uint64_t half = uint64_t(1) << k;
+        for (uint64_t i = threadIdx.x; i < entries; i += blockDim.x) {
+            uint2 e = __ldcg(src + 2u * i);
+            if ((i << s) + half < w.n) e = win_first(e, __ldcg(src + 2u * i + wpu), w.wide ? uint32_t(half) : 0u);
+            dst[i] = e;
+        }
+        __syncthreads();
+    }
+}
+
+}  // namespace rmq

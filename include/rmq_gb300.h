@@ -47,23 +47,24 @@ typedef enum {
 } rmq_status;
 
 typedef enum {
-    RMQ_VARIANT_AUTO = 0,  /* the measured best: VL with rf = 8                                          */
+    RMQ_VARIANT_AUTO = 0,  /* the measured best: VL                                                       */
     RMQ_VARIANT_CL = 1,    /* tile of lanes answering its queries one after another (reference alg 16 family) */
-    RMQ_VARIANT_VL = 2,    /* one thread per query, 256-bit loads (reference alg 20 family)              */
+    RMQ_VARIANT_VL = 2,    /* 256-bit loads, a thread per query (reference alg 20 family), over window tables:
+                              a query takes the two windows that cover it and, when their first minimum lies
+                              outside it, the exact answer from windows and blocks inside it              */
     /* The reference's ablations of its CL kernel: the same hierarchy and
      * results, other work distributions (src/xxx.h:302-790). */
     RMQ_VARIANT_CL_NO_SHUFFLE = 3,     /* each lane loads the turn's query itself (alg 23)              */
     RMQ_VARIANT_CL_QUERY_PER_TILE = 4, /* one query per tile of lanes, no turns (alg 24)               */
     RMQ_VARIANT_CL_ATOMIC = 5,         /* lanes combine with atomic minima, no shuffle reduction (alg 19);
                                           scan threshold below 2^27                                      */
-    /* VL for workloads of short queries (rf 8, 32-bit positions; otherwise
-     * VL): a query of at most 512 entries takes its level-0 winner while it
-     * folds level 0 instead of reading that sector again to locate it, which
-     * its evict-first L2 line seldom survives.  Same results. */
+    /* The same as VL (the name of an earlier form for short queries). */
     RMQ_VARIANT_VL_SHORT = 6
 } rmq_variant;
 
 typedef struct {
+    /* t and rf plan the levels that CL handles hold and rmq_get_info reports;
+     * a VL handle checks and reports them, its window tables do not depend on them. */
     int32_t  variant;         /* rmq_variant                                                    */
     uint64_t scan_threshold;  /* t: build levels while a level holds more than t entries (0 = variant default) */
     int32_t  rf_log;          /* log2 of the per-level reduction factor, 3..5 (0 = variant default)       */
@@ -83,7 +84,8 @@ typedef struct {
     uint64_t scan_threshold;    /* resolved t                                            */
     uint64_t level_size[20];    /* entries per level                                     */
     uint64_t level_offset[20];  /* element offset of level k >= 1 in the level buffer    */
-    uint64_t level_bytes;       /* device bytes of level values (+ argmin arrays)        */
+    uint64_t level_bytes;       /* device bytes of level values (+ argmin arrays); a VL handle's window
+                                   tables take no more (n > 64)                           */
     float    build_ms;          /* device time of the last build (CUDA events)           */
     int32_t  index_bits;        /* 32 or 64                                              */
 } rmq_info;
@@ -171,8 +173,8 @@ const char* rmq_strerror(int status);
  * cudaMalloc / cudaFree are off limits because those calls can block and
  * synchronise the device.  It has no counterpart in the reference.
  *
- * The hierarchy (VL, rf = 8, scan threshold t; 0 = 32) is built into one
- * fixed 8 MiB device array owned by the library, which every GPU that loads
+ * The window tables (t, the scan threshold, is checked as rmq_build checks
+ * it; 0 = 32) are built into one fixed 8 MiB device array owned by the library, which every GPU that loads
  * the library holds until the process exits; then the queries are answered,
  * both on `stream`.  Limit: n <= 2^22 (4,194,304 entries); a larger n, or a t
  * whose levels do not fit, returns RMQ_ERR_UNSUPPORTED before any device

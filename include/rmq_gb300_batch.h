@@ -4,11 +4,13 @@
  *
  * The reference answers one array per run of its driver (src/main.cu:71-287),
  * so a workload of thousands of arrays is a loop of builds and query launches
- * (src/xxx.h:258-281 per array).  A batch packs the arrays' coarse levels in
- * one allocation, builds all of them with two kernels, answers all their
+ * (src/xxx.h:258-281 per array).  A batch packs the arrays' tables in one
+ * allocation, builds all of them with two to four kernels, answers all their
  * query sets with one kernel, and can replay build + queries as one CUDA
  * graph launch.  Semantics per query are exactly those of rmq_query_idx
- * (include/rmq_gb300.h).  The work distribution is VL with rf = 8.
+ * (include/rmq_gb300.h).  The arrays hold VL's window tables; the scan
+ * thresholds below plan the levels that rmq_batch_info reports (rf 8) and do
+ * not change the tables.
  */
 #ifndef RMQ_GB300_BATCH_H
 #define RMQ_GB300_BATCH_H
@@ -56,7 +58,7 @@ int rmq_batch_create(const float* d_values, const uint64_t* value_offsets, const
 int rmq_batch_set_queries(rmq_batch* b, const uint32_t* d_lr, const uint64_t* query_offsets,
                           uint32_t* d_argmin, float* d_min, rmq_stream_t stream);
 
-/* Enqueues the build of every array's coarse levels (two kernel launches). */
+/* Enqueues the build of every array's tables (two to four kernel launches). */
 int rmq_batch_build(rmq_batch* b, rmq_stream_t stream);
 
 /* Enqueues one query launch over every registered query of every array. */
@@ -75,13 +77,10 @@ int rmq_batch_run(rmq_batch* b, rmq_stream_t stream);
  * are identical to rmq_batch_run's. */
 int rmq_batch_run_per_array(rmq_batch* b, rmq_stream_t stream);
 
-/* Autotuner: times the query kernel on the registered queries for each
- * candidate scan threshold t in {16, 32, 64, 256, 1024} (the same for every
- * array) and CTA size in {64, 128, 256, 512} threads; then, keeping the best
- * CTA size, tries each t for each array-size class in turn (arrays below 2^14
- * entries, below 2^18, and the rest; the largest class first) and keeps a
- * class's new t when it is faster by more than 0.5 %.  Rebuilds with the
- * choice.  Blocking.  The choice is reported in *info (may be NULL). */
+/* Autotuner: times the query kernel on the registered queries for each CTA
+ * size in {64, 128, 256, 512} threads, keeps the best and rebuilds.  A size
+ * class's threshold that is not one of {16, 32, 64, 256, 1024} becomes 64.
+ * Blocking.  The choice is reported in *info (may be NULL). */
 int rmq_batch_autotune(rmq_batch* b, rmq_stream_t stream, rmq_batch_info* info);
 
 /* Applies a known choice (for example one rmq_batch_autotune made earlier for
