@@ -43,7 +43,7 @@ batch_block_kernel(const float* __restrict__ values, const ArrayDesc* __restrict
     win_block_tile(w, tile);
 }
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kLowThreads)
 batch_low_kernel(const ArrayDesc* __restrict__ descs, TileList l, char* tables) {
     __shared__ uint2 sa[kSpan + kHaloLow], sb[kSpan + kHaloLow];
     WinOut w;
@@ -51,7 +51,7 @@ batch_low_kernel(const ArrayDesc* __restrict__ descs, TileList l, char* tables) 
     win_low_tile(w, tile, sa, sb);
 }
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kMidThreads)
 batch_mid_kernel(const ArrayDesc* __restrict__ descs, TileList l, char* tables) {
     __shared__ uint2 sa[kSpan + kHaloMid], sb[(kSpan + kHaloMid) / 2];
     WinOut w;
@@ -59,11 +59,12 @@ batch_mid_kernel(const ArrayDesc* __restrict__ descs, TileList l, char* tables) 
     win_mid_tile(w, tile, sa, sb);
 }
 
-__global__ void __launch_bounds__(1024)
+__global__ void __launch_bounds__(kMidThreads)
 batch_top_kernel(const ArrayDesc* __restrict__ descs, TileList l, char* tables) {
+    __shared__ uint2 sa[kTopEntries], sb[kTopEntries / 2];
     WinOut w;
     batch_tile(descs, l, nullptr, tables, w);
-    win_top(w);
+    win_top(w, sa, sb);
 }
 
 // Work unit of the query kernels: consecutive queries of one array, answered by
@@ -333,9 +334,9 @@ cudaError_t enqueue_build(rmq_batch* b, cudaStream_t s) {
     const auto list = [&](int i) { return rmq::TileList{w[i].d_off, w[i].d_owner}; };
     rmq::batch_block_kernel<<<uint32_t(w[0].total), rmq::kBlockThreads, 0, s>>>(b->d_values, b->d_descs, list(0),
                                                                                b->tables);
-    if (w[1].total > 0) rmq::batch_low_kernel<<<uint32_t(w[1].total), 256, 0, s>>>(b->d_descs, list(1), b->tables);
-    if (w[2].total > 0) rmq::batch_mid_kernel<<<uint32_t(w[2].total), 256, 0, s>>>(b->d_descs, list(2), b->tables);
-    if (w[3].total > 0) rmq::batch_top_kernel<<<uint32_t(w[3].total), 1024, 0, s>>>(b->d_descs, list(3), b->tables);
+    if (w[1].total > 0) rmq::batch_low_kernel<<<uint32_t(w[1].total), rmq::kLowThreads, 0, s>>>(b->d_descs, list(1), b->tables);
+    if (w[2].total > 0) rmq::batch_mid_kernel<<<uint32_t(w[2].total), rmq::kMidThreads, 0, s>>>(b->d_descs, list(2), b->tables);
+    if (w[3].total > 0) rmq::batch_top_kernel<<<uint32_t(w[3].total), rmq::kMidThreads, 0, s>>>(b->d_descs, list(3), b->tables);
     return cudaGetLastError();
 }
 

@@ -17,23 +17,24 @@ __global__ void __launch_bounds__(kBlockThreads) win_block_kernel(WinOut w) {
     win_block_tile(w, blockIdx.x);
 }
 
-__global__ void __launch_bounds__(256) win_low_kernel(WinOut w) {
+__global__ void __launch_bounds__(kLowThreads) win_low_kernel(WinOut w) {
     __shared__ uint2 sa[kSpan + kHaloLow], sb[kSpan + kHaloLow];
     wait_previous_grid();
     allow_next_grid();
     win_low_tile(w, blockIdx.x, sa, sb);
 }
 
-__global__ void __launch_bounds__(256) win_mid_kernel(WinOut w) {
+__global__ void __launch_bounds__(kMidThreads) win_mid_kernel(WinOut w) {
     __shared__ uint2 sa[kSpan + kHaloMid], sb[(kSpan + kHaloMid) / 2];
     wait_previous_grid();
     allow_next_grid();
     win_mid_tile(w, blockIdx.x, sa, sb);
 }
 
-__global__ void __launch_bounds__(1024) win_top_kernel(WinOut w) {
+__global__ void __launch_bounds__(kMidThreads) win_top_kernel(WinOut w) {
+    __shared__ uint2 sa[kTopEntries], sb[kTopEntries / 2];
     wait_previous_grid();
-    win_top(w);
+    win_top(w, sa, sb);
 }
 
 // Launch with programmatic stream serialization (the kernel waits for its
@@ -74,9 +75,9 @@ cudaError_t launch_window_build(const float* d_values, void* tables, uint64_t n,
     const WinTiles t = win_tiles(sh);
     win_block_kernel<<<uint32_t(t.block), kBlockThreads, 0, s>>>(w);
     cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess && t.low > 0) e = launch_dependent(win_low_kernel, uint32_t(t.low), 256, s, w);
-    if (e == cudaSuccess && t.mid > 0) e = launch_dependent(win_mid_kernel, uint32_t(t.mid), 256, s, w);
-    if (e == cudaSuccess && t.top > 0) e = launch_dependent(win_top_kernel, uint32_t(t.top), 1024, s, w);
+    if (e == cudaSuccess && t.low > 0) e = launch_dependent(win_low_kernel, uint32_t(t.low), kLowThreads, s, w);
+    if (e == cudaSuccess && t.mid > 0) e = launch_dependent(win_mid_kernel, uint32_t(t.mid), kMidThreads, s, w);
+    if (e == cudaSuccess && t.top > 0) e = launch_dependent(win_top_kernel, uint32_t(t.top), kMidThreads, s, w);
     return e;
 }
 

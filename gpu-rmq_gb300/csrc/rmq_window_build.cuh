@@ -16,9 +16,12 @@ namespace rmq {
 
 constexpr uint32_t kBlockTile = 8192;      // level-0 entries per CTA of the block pass
 constexpr uint32_t kBlockThreads = 256;
+constexpr uint32_t kLowThreads = 512;
+constexpr uint32_t kMidThreads = 1024;
 constexpr uint32_t kSpan = 2048;           // own strides per tile of the window kernels
 constexpr uint32_t kHaloLow = 512;         // halo of the first window kernel, in strides of 2^gb
 constexpr uint32_t kHaloMid = 1024;        // halo of the second, in its input's strides
+constexpr uint32_t kTopEntries = 4096;     // entries of T_(gb+15) the last kernel holds in shared memory
 constexpr uint32_t kMidSteps = 6;          // sizes the second window kernel adds
 
 // Largest window the first kernel makes from a tile and its halo (512 strides
@@ -136,45 +139,74 @@ __device__ __forceinline__ void win_double_up(const WinOut& w, uint32_t k, uint3
     }
 }
 
-// The tables up to T_(gb+9) (all of them when the array has one tile) of the
-// tile's kSpan strides of 2^gb entries.
-__device__ __forceinline__ void win_low_tile(const WinOut& w, uint64_t tile, uint2* sa, uint2* sb) {
-    const uint64_t g0 = tile * kSpan;
-    const uint32_t cnt = kSpan + kHaloLow;
-    const uint32_t bpg = 1u << (w.gb - w.blk);  // blocks per stride
-    const uint64_t nb = (w.n + (uint64_t(1) << w.blk) - 1) >> w.blk;
-    for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) {
-        if (g0 + i >= w.S) break;
-        const uint64_t b = (g0 + i) * bpg;
-        uint2 e = make_uint2(__float_as_uint(w.v1[b]), w.j1[b]);
-        for (uint32_t c = 1; c < bpg; ++c)
-            if (b + c < nb) e = win_first(e, make_uint2(__float_as_uint(w.v1[b + c]), w.j1[b + c]), c << w.blk);
-        if (!w.wide) e.y += uint32_t(b << w.blk);
-        sa[i] = e;
+// First minimum of the blocks of stride g (g < S), as an entry of T.
+__device__ __forceinline__ uint2 win_group(const WinOut& w, uint64_t g) {
+    const uint32_t bpg = 1u << (w.gb - w.blk);  // blocks per stride: 2 or 4
+    const uint64_t nb = (w.n + (uint64_t(1) << w.blk) - 1) >> w.blk, b = g * bpg;
+    float v[4];
+    uint32_t off;
+    // V1 and J1 are padded to 32 bytes, so a whole stride of either can be read
+    if (bpg == 2u) {
+        const float2 x = *reinterpret_cast<const float2*>(w.v1 + b);
+        v[0] = x.x;
+        v[1] = x.y;
+        v[2] = v[3] = f_inf();
+        off = *reinterpret_cast<const uint16_t*>(w.j1 + b);
+    } else {
+        const float4 x = *reinterpret_cast<const float4*>(w.v1 + b);
+        v[0] = x.x;
+        v[1] = x.y;
+        v[2] = x.z;
+        v[3] = x.w;
+        off = *reinterpret_cast<const uint32_t*>(w.j1 + b);
     }
-    __syncthreads();
+    uint2 e = make_uint2(__float_as_uint(v[0]), off & 255u);
+#pragma unroll
+    for (uint32_t c = 1; c < 4; ++c)
+        if (c < bpg && b + c < nb) e = win_first(e, make_uint2(__float_as_uint(v[c]), (off >> (8u * c)) & 255u), c << w.blk);
+    if (!w.wide) e.y += uint32_t(b << w.blk);
+    return e;
+}
+
+// The tables up to T_(gb+9) (all of them when the array has one tile) of the
+// tile's kSpan strides of 2^gb entries, by kLowThreads threads.  A tile is a
+// chain of some ten steps with a barrier each, so its time is their latency:
+// every thread keeps its entries in registers, all loads of a step in flight
+// (one tile: 16 -> 8.5 us against one entry after another with 256 threads;
+// the build of 2^20 values 25 -> 19 us, of 2^26 80 -> 71 us).
+__device__ __forceinline__ void win_low_tile(const WinOut& w, uint64_t tile, uint2* sa, uint2* sb) {
+    constexpr uint32_t kPer = (kSpan + kHaloLow) / kLowThreads;
+    const uint64_t g0 = tile * kSpan;
+    uint2 e[kPer];
+#pragma unroll
+    for (uint32_t u = 0; u < kPer; ++u) {
+        const uint64_t g = g0 + threadIdx.x + kLowThreads * u;
+        if (g < w.S) e[u] = win_group(w, g);
+    }
     // Windows of 2, 4, 8 strides (2^first entries), the last one the first
     // table; where the next one has the same stride, a doubling of 8.
     uint2 *src = sa, *dst = sb;
     const uint32_t kb = w.gb + w.c;
-    for (uint32_t d = 1; d <= (w.first < kb ? 8u : 4u); d <<= 1) {
+    for (uint32_t d = 1;; d <<= 1) {
+#pragma unroll
+        for (uint32_t u = 0; u < kPer; ++u) src[threadIdx.x + kLowThreads * u] = e[u];
+        __syncthreads();
+        if (d > (w.first < kb ? 8u : 4u)) break;
         uint2* out = nullptr;
         if (d == 4u) out = w.t + win_table_at<uint64_t>(w, w.first) + g0;
         if (d == 8u && w.kmax >= kb) out = w.t + win_table_at<uint64_t>(w, kb) + g0;
-        for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) {
-            if (g0 + i >= w.S) break;
-            uint2 e = src[i];
-            if (i + d < cnt && g0 + i + d < w.S) e = win_first(e, src[i + d], w.wide ? d << w.gb : 0u);
-            dst[i] = e;
-            if (out != nullptr && i < kSpan) out[i] = e;
+#pragma unroll
+        for (uint32_t u = 0; u < kPer; ++u) {
+            const uint32_t i = threadIdx.x + kLowThreads * u;
+            if (g0 + i + d < w.S && i + d < kSpan + kHaloLow) e[u] = win_first(e[u], src[i + d], w.wide ? d << w.gb : 0u);
+            if (out != nullptr && i < kSpan && g0 + i < w.S) out[i] = e[u];
         }
-        __syncthreads();
         uint2* x = src;
         src = dst;
         dst = x;
     }
     const uint32_t last = w.S <= kSpan ? w.kmax : (w.kmax < win_low_log(w) ? w.kmax : win_low_log(w));
-    win_double_up(w, kb, last, g0, cnt, kSpan, src, dst);
+    win_double_up(w, kb, last, g0, kSpan + kHaloLow, kSpan, src, dst);
 }
 
 // The next kMidSteps tables above T_(gb+9) of one tile of its entries.
@@ -184,10 +216,15 @@ __device__ __forceinline__ void win_mid_tile(const WinOut& w, uint64_t tile, uin
     const uint32_t cnt = kSpan + kHaloMid;
     const uint64_t entries = (w.n + (uint64_t(1) << s) - 1) >> s;
     const uint2* src = w.t + win_table_at<uint64_t>(w, k) + e0;
-    for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) {
-        if (e0 + i >= entries) break;
-        sa[i] = __ldcg(src + i);
+    constexpr uint32_t kPer = (kSpan + kHaloMid) / kMidThreads;
+    uint2 e[kPer];
+#pragma unroll
+    for (uint32_t u = 0; u < kPer; ++u) {
+        const uint32_t i = threadIdx.x + kMidThreads * u;
+        if (e0 + i < entries) e[u] = __ldcg(src + i);
     }
+#pragma unroll
+    for (uint32_t u = 0; u < kPer; ++u) sa[threadIdx.x + kMidThreads * u] = e[u];
     __syncthreads();
     const uint32_t last = entries <= kSpan ? w.kmax : (w.kmax < win_mid_log(w) ? w.kmax : win_mid_log(w));
     win_double_up(w, k, last, e0, cnt, kSpan, sa, sb);
@@ -208,11 +245,25 @@ inline WinTiles win_tiles(const WinShape& w) {
     return t;
 }
 
-// The tables above T_(gb+15), by one CTA (at 2^26 entries: 512 entries and
-// halving), each from the one below in global memory.
-__device__ __forceinline__ void win_top(const WinOut& w) {
+// The tables above T_(gb+15), by one CTA of kMidThreads: from shared memory
+// where its entries fit there (up to 2^28 entries), else each table from the
+// one below in global memory.
+__device__ __forceinline__ void win_top(const WinOut& w, uint2* sa, uint2* sb) {
+    const uint32_t k0 = win_mid_log(w), s0 = win_stride_log(w, k0);
+    const uint64_t have = (w.n + (uint64_t(1) << s0) - 1) >> s0;
+    const uint2* from = w.t + win_table_at<uint64_t>(w, k0);
+    if (have <= kTopEntries) {
+#pragma unroll
+        for (uint32_t u = 0; u < kTopEntries / kMidThreads; ++u) {
+            const uint32_t i = threadIdx.x + kMidThreads * u;
+            if (i < have) sa[i] = __ldcg(from + i);
+        }
+        __syncthreads();
+        win_double_up(w, k0, w.kmax, 0, kTopEntries, kTopEntries, sa, sb);
+        return;
+    }
     const uint32_t wpu = 1u << w.c;
-    for (uint32_t k = win_mid_log(w); k < w.kmax; ++k) {
+    for (uint32_t k = k0; k < w.kmax; ++k) {
         const uint32_t s = win_stride_log(w, k + 1u);
         const uint64_t entries = (w.n + (uint64_t(1) << s) - 1) >> s;
         const uint2* src = w.t + win_table_at<uint64_t>(w, k);
