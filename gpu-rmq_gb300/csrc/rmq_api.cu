@@ -39,6 +39,8 @@ struct rmq_handle {
     std::mutex validate_mu;
 
     bool windows() const { return variant == RMQ_VARIANT_VL || variant == RMQ_VARIANT_VL_SHORT; }
+    // Positions may be asked for (without argmin arrays only when the plan is level 0 alone).
+    bool positions() const { return with_index != 0 || lay.num_levels == 1; }
 
     // Staging of the host-buffer calls (rmq_query_host / rmq_query_idx_host),
     // created on the first such call.
@@ -236,7 +238,7 @@ int rmq_build(const float* d_values, uint64_t n, const rmq_config* cfg, rmq_stre
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     cudaError_t e = cudaSuccess;
     if (h->windows()) {
-        h->level_bytes = rmq::window_bytes(n, h->with_index != 0);
+        h->level_bytes = rmq::window_bytes(n, h->positions());
         e = cudaMalloc(&h->tables, h->level_bytes);
     } else if (h->lay.num_levels > 1) {
         // One allocation: level values, then argmin indices, so that a single
@@ -262,7 +264,7 @@ int rmq_build(const float* d_values, uint64_t n, const rmq_config* cfg, rmq_stre
     if (e == cudaSuccess) e = cudaEventCreate(&e1);
     if (e == cudaSuccess) e = cudaEventRecord(e0, s);
     if (e == cudaSuccess)
-        e = h->windows() ? rmq::launch_window_build(d_values, h->tables, n, h->with_index != 0, wide, s)
+        e = h->windows() ? rmq::launch_window_build(d_values, h->tables, n, h->positions(), wide, s)
                          : rmq::launch_build(h->lay, d_values, h->val_buf, h->idx_buf, s, h->counters);
     if (e == cudaSuccess) e = cudaEventRecord(e1, s);
     if (e == cudaSuccess) e = cudaEventSynchronize(e1);
@@ -303,8 +305,8 @@ static rmq::QueryArgs query_args(const rmq_handle* h, const void* d_lr, uint64_t
     rmq::QueryArgs a;
     std::memset(&a, 0, sizeof(a));
     if (h->windows()) {
-        if (h->wide) a.win64 = rmq::win_view<uint64_t>(h->d_values, h->tables, h->lay.n, h->with_index != 0);
-        else a.win = rmq::win_view<uint32_t>(h->d_values, h->tables, h->lay.n, h->with_index != 0);
+        if (h->wide) a.win64 = rmq::win_view<uint64_t>(h->d_values, h->tables, h->lay.n, h->positions());
+        else a.win = rmq::win_view<uint32_t>(h->d_values, h->tables, h->lay.n, h->positions());
     } else {
         for (uint32_t k = 0; k < h->lay.num_levels; ++k) {
             a.lv.val[k] = k == 0 ? h->d_values : h->val_buf + h->lay.offset[k];
@@ -346,7 +348,7 @@ static int query_common(const rmq_handle* hc, const void* d_lr, uint64_t q, floa
     if ((reinterpret_cast<uintptr_t>(d_min) & 3u) != 0 ||
         (reinterpret_cast<uintptr_t>(d_argmin) & (wide_call ? 7u : 3u)) != 0)
         return RMQ_ERR_ARG;
-    if (d_argmin != nullptr && !hc->with_index && hc->lay.num_levels > 1) return RMQ_ERR_NO_INDEX;
+    if (d_argmin != nullptr && !hc->positions()) return RMQ_ERR_NO_INDEX;
     rmq_handle* h = const_cast<rmq_handle*>(hc);
     DeviceGuard guard(h->device);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
@@ -461,7 +463,7 @@ static int query_host_common(const rmq_handle* hc, const void* h_lr, uint64_t q,
     if (q == 0) return RMQ_OK;
     if (!wide_call && q > 0xFFFFFFFFull) return RMQ_ERR_UNSUPPORTED;
     if (h_lr == nullptr || (h_min == nullptr && h_argmin == nullptr)) return RMQ_ERR_ARG;
-    if (h_argmin != nullptr && !hc->with_index && hc->lay.num_levels > 1) return RMQ_ERR_NO_INDEX;
+    if (h_argmin != nullptr && !hc->positions()) return RMQ_ERR_NO_INDEX;
     rmq_handle* h = const_cast<rmq_handle*>(hc);
     DeviceGuard guard(h->device);
     rmq_handle::HostPipe& p = h->pipe;

@@ -94,40 +94,41 @@ uint64_t window_bytes(uint64_t n, bool with_index) {
 // for the others.  n = 2^20, device time of one launch in us, the two kernels
 // and the block-minimum descent they replace:
 //
-//   queries                2^18               2^20                2^22
-//   uniform lengths     8.0  10.8  14.0   15.7  33.1  38.6    38.3  119  137
-//   lognormal(2^13, 1) 10.1  10.7  12.7   17.4  29.8  34.0    47.9  106  119
-//   lognormal(32, 0.7) 12.3   8.7   8.6   27.7  22.7  22.9    86.7   80   82
+//   queries                2^18               2^20               2^22
+//   uniform lengths      7.8   8.9  14.2   14.6  23.1  38.7   37.4  119  138
+//   lognormal(2^13, 1)   8.7   9.0  13.0   16.3  23.9  34.1   41.1  106  120
+//   lognormal(32, 0.7)  10.9   9.2   8.6   25.2  24.6  23.1   81.6   80   83
+//   all three mixed     11.4  13.1  14.3   24.0  36.5  38.9   66.1        141
 //
-// The lengths are not known before the launch.  win_one_kernel answers up to
-// 2^18 queries, and up to 2^20 over a small array (blocks of eight entries),
-// where short queries are fast enough to notice the lists; at n = 2^26 the
-// lists win for every law from 2^19 on.  Results in host memory always come
-// from win_one_kernel: its warps write whole 128-byte lines, which the
+// The lengths are not known before the launch: win_one_kernel answers up to
+// 2^18 queries, where it is the faster one only for short lengths but never
+// slower than the descent by more than a few percent.  Results in host memory
+// always come from it: its warps write whole 128-byte lines, which the
 // CPU-GPU link wants (2^22 queries, page-locked: 214 us against 385).
 //
 // kQueryThreads and the blocks per SM: the loads in flight live in the part
 // of the SM's 256 KiB that shared memory leaves (8 KiB per block here); with
 // 16 KiB per block, or 32 KiB of shared memory more in all, the headline
 // workload (lognormal(2^13, 1), n = q = 2^26) takes 6 % to 100 % longer.
+// Without positions ten blocks fit without spills (short queries 4 to 6 %
+// faster); with them ten spill 40 bytes (the headline workload 717 -> 779 us).
 constexpr uint32_t kQueryThreads = 128;
 constexpr uint32_t kLaneQueries = 4;
 constexpr uint32_t kBlockQueries = kQueryThreads * kLaneQueries;
 constexpr uint32_t kOneThreads = 64;
 constexpr uint64_t kFewQueries = uint64_t(1) << 18;
-constexpr uint64_t kFewQueriesSmall = uint64_t(1) << 20;
 
-template <bool ARGMIN, typename I>
-__global__ void __launch_bounds__(kQueryThreads, sizeof(I) == 4 ? 9 : 8)
+template <bool ARGMIN, bool COLD, typename I>
+__global__ void __launch_bounds__(kQueryThreads, sizeof(I) == 4 ? (ARGMIN ? 9 : 10) : 8)
 win_query_kernel(WinViewT<I> w, const typename IdxTraits<I>::Pair* __restrict__ qs, uint64_t q,
                  float* __restrict__ out_min, I* __restrict__ out_idx, uint32_t* __restrict__ err) {
     __shared__ __align__(16) unsigned char smem[win_lists_bytes<I>(kBlockQueries)];
     const uint64_t at = uint64_t(blockIdx.x) * kBlockQueries;
     const uint32_t cnt = q - at < kBlockQueries ? uint32_t(q - at) : kBlockQueries;
     const WinLists<I> sm = win_lists<I>(smem, kBlockQueries);
-    const uint32_t bad = win_block<ARGMIN, kLaneQueries>(w, sm, kQueryThreads, qs + at, cnt,
-                                                         out_min != nullptr ? out_min + at : nullptr,
-                                                         ARGMIN ? out_idx + at : nullptr);
+    const uint32_t bad = win_block<ARGMIN, COLD, kLaneQueries>(w, sm, kQueryThreads, qs + at, cnt,
+                                                               out_min != nullptr ? out_min + at : nullptr,
+                                                               ARGMIN ? out_idx + at : nullptr);
     if (bad != 0u && err != nullptr) atomicAdd(err, bad);
 }
 
@@ -154,11 +155,12 @@ win_one_kernel(WinViewT<I> w, const typename IdxTraits<I>::Pair* __restrict__ qs
 template <bool ARGMIN, typename I>
 static cudaError_t launch_window_typed(const QueryArgs& a, const WinViewT<I>& w,
                                        const typename IdxTraits<I>::Pair* qs, I* out_idx, cudaStream_t s) {
-    if (a.q <= (w.n <= kSmallN ? kFewQueriesSmall : kFewQueries) || a.host_buffers)
+    if (a.q <= kFewQueries || a.host_buffers)
         return launch_with_window(win_one_kernel<ARGMIN, I>, uint32_t((a.q + kOneThreads - 1u) / kOneThreads), kOneThreads,
                                   a, s, w, qs, a.q, a.out_min, out_idx, a.err);
-    return launch_with_window(win_query_kernel<ARGMIN, I>, uint32_t((a.q + kBlockQueries - 1u) / kBlockQueries),
-                              kQueryThreads, a, s, w, qs, a.q, a.out_min, out_idx, a.err);
+    return launch_with_window(w.n > kWarmN ? win_query_kernel<ARGMIN, true, I> : win_query_kernel<ARGMIN, false, I>,
+                              uint32_t((a.q + kBlockQueries - 1u) / kBlockQueries), kQueryThreads, a, s, w, qs, a.q,
+                              a.out_min, out_idx, a.err);
 }
 
 cudaError_t launch_window_query(const QueryArgs& a, cudaStream_t s) {

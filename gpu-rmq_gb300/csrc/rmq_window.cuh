@@ -26,15 +26,16 @@
 // in 23 (c = 4) or 12 (c = 3); then the query is answered exactly, from
 // windows and blocks that lie inside it, with the two blocks at its ends read
 // at level 0 only when their minimum would win (win_exact).  A shorter query
-// takes the first minimum of the blocks that touch it in the same way.
+// is answered from its blocks: the ones inside it and its ends (win_short), or
+// by the cover of the blocks that touch it where level 0 is in DRAM.
 //
 // Measured, min + argmin, against the block-minimum descent (one thread per
 // query, rf = 8) that it replaces, us per launch: lognormal(2^13, 1) lengths,
-// n = q = 2^26: 2567 -> 720; the mixture of three length laws with 1 % of the
-// values at the minimum, n = q = 2^26: 3377 -> 1637, n = 2^28, q = 2^27:
-// 9962 -> 4870; uniform lengths, minima, n = 5e7, q = 3e7: 1226 -> 250;
-// lognormal(32, 0.7), positions, n = 2^26, q = 2^25: 1370 -> 701; 64-bit
-// positions, lognormal(2^13, 1), n = 2^26, q = 2^25: 1503 -> 571.
+// n = q = 2^26: 2567 -> 718; the mixture of three length laws with 1 % of the
+// values at the minimum, n = q = 2^26: 3377 -> 1617, n = 2^28, q = 2^27:
+// 9962 -> 4853; uniform lengths, minima, n = 5e7, q = 3e7: 1226 -> 240;
+// lognormal(32, 0.7), positions, n = 2^26, q = 2^25: 1370 -> 698; 64-bit
+// positions, lognormal(2^13, 1), n = 2^26, q = 2^25: 1503 -> 567.
 #pragma once
 
 #include "rmq_common.cuh"
@@ -43,21 +44,23 @@ namespace rmq {
 
 // Sizes of the tables: log2 of the block, of the smallest stride, of the
 // strides per window (from window 2^(gb + c) on; smaller ones keep the
-// smallest stride), and of the first window.  Up to 2^22 entries, where
-// everything stays in L2 and short queries are bound by instructions, blocks
-// of eight entries (one sector; a cover of 32 entries fails for a fifth of the
-// queries instead of a third) and windows at every eighth of their size;
-// beyond, blocks of 16 keep V1 in L2 (length 32, q = 2^22, us: n = 2^20
-// 76 against 97 with blocks of 16).  Bytes per value: 1.125 up to 2^22, then
-// 1.0625, and 0.5625 without argmin; the block-minimum levels with their
-// stored indices take 1.143 and 0.571, so what fitted before still fits.
+// smallest stride), and of the first window.  Bytes per value: 1.0625 with
+// argmin, without 0.5625, and 1.125 up to 2^22 entries; the block-minimum
+// levels with their stored indices take 1.143 and 0.571, so what fitted before
+// still fits.  Windows at every 16th of their size fail half as often as at
+// every 8th, which counts for more than short queries do: with blocks of
+// eight entries and c = 3 for argmin too, 384 arrays of 2^10 .. 2^20 values
+// built and queried together take 2149 us instead of 1960, and n = 2^20, q =
+// 2^22, us, length 24: 65 instead of 75, lognormal(2^13, 1): 48 instead of 41.
+// Without argmin blocks of eight pay for small arrays, whose short queries are
+// bound by instructions (length 24: 52 us, with blocks of 16: 67).
 struct WinForm {
     uint32_t blk, gb, c, first;
 };
 constexpr uint64_t kSmallN = uint64_t(1) << 22;
 __host__ __device__ inline WinForm win_form(uint64_t n, bool with_index) {
-    if (n <= kSmallN) return WinForm{3, 5, 3, 8};
-    return with_index ? WinForm{4, 5, 4, 8} : WinForm{4, 6, 3, 9};
+    if (with_index) return WinForm{4, 5, 4, 8};
+    return n <= kSmallN ? WinForm{3, 5, 3, 8} : WinForm{4, 6, 3, 9};
 }
 constexpr uint32_t kMaxWinLog = 32;  // largest window (offsets are 32-bit)
 
@@ -279,10 +282,10 @@ __device__ __forceinline__ WinBest<I> win_none() {
 __device__ __forceinline__ uint32_t win_bits(uint32_t lo, uint32_t hi) { return ((1u << hi) - 1u) & ~((1u << lo) - 1u); }
 
 __device__ __forceinline__ float win_pick(const float (&v)[8], uint32_t j) {
-    float x = v[0];
-#pragma unroll
-    for (int t = 1; t < 8; ++t) x = (j == uint32_t(t)) ? v[t] : x;
-    return x;
+    const bool b0 = (j & 1u) != 0u, b1 = (j & 2u) != 0u;
+    const float x0 = b0 ? v[1] : v[0], x1 = b0 ? v[3] : v[2], x2 = b0 ? v[5] : v[4], x3 = b0 ? v[7] : v[6];
+    const float y0 = b1 ? x1 : x0, y1 = b1 ? x3 : x2;
+    return (j & 4u) != 0u ? y1 : y0;
 }
 
 // v[j] where bit j of `mask` is set, else +inf; the minimum of those.
@@ -290,6 +293,16 @@ __device__ __forceinline__ float win_mask8(float (&v)[8], uint32_t mask) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) v[j] = ((mask >> j) & 1u) != 0u ? v[j] : f_inf();
     return fmin3(fmin3(v[0], v[1], v[2]), fmin3(v[3], v[4], v[5]), fminf(v[6], v[7]));
+}
+
+// The minimum of v[j] over the bits of `mask`, where its place is not wanted
+// (a predicated min per entry: 3 % faster than win_mask8 there).
+__device__ __forceinline__ float win_min8(const float (&v)[8], uint32_t mask) {
+    float m = f_inf();
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+        if ((mask & (1u << j)) != 0u) m = fminf(m, v[j]);
+    return m;
 }
 
 // First entry of u equal to x, their minimum (not NaN), and in x its own bits.
@@ -360,6 +373,36 @@ __device__ __forceinline__ void ld_values8(const WinViewT<I>& w, I s, float (&v)
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[j] = (s + I(j) < w.n) ? w.a[s + j] : f_inf();
     }
+}
+
+// The same loads where `p` holds, zeros elsewhere (the caller masks them out);
+// a sector of level 0 has to lie inside the array.  Without the zeros the
+// registers of a load that may not happen count as live from the start of the
+// kernel, and it spills 176 bytes.
+template <typename I>
+__device__ __forceinline__ void ld_blocks8_if(const WinViewT<I>& w, bool p, I b, float (&v)[8]) {
+#if RMQ_DEBUG_BOUNDS
+    p = p && bounds_ok((b & 7u) == 0 && (b << w.blk) < w.n);
+#endif
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = 0.0f;
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %10, 0;\n\t"
+        "@p ld.global.nc.L2::cache_hint.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8], %9;\n\t}"
+        : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7])
+        : "l"(w.v1 + b), "l"(policy_evict_last()), "r"(uint32_t(p)));
+}
+
+template <typename I>
+__device__ __forceinline__ void ld_values8_if(const WinViewT<I>& w, bool p, I s, float (&v)[8]) {
+#if RMQ_DEBUG_BOUNDS
+    p = p && bounds_ok((s & 7u) == 0 && s + 8u <= w.n);
+#endif
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = 0.0f;
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %10, 0;\n\t"
+        "@p ld.global.nc.L2::cache_hint.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8], %9;\n\t}"
+        : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7])
+        : "l"(w.a + s), "l"(policy_evict_first()), "r"(uint32_t(p)));
 }
 
 // First minimum of level-0 entries [lo, hi) (lo < hi), which touch at most N
@@ -464,6 +507,156 @@ __device__ __forceinline__ bool win_short_cover(const WinViewT<I>& w, I l, I R, 
     cur.p = (cur.p << w.blk) + ld_block_off(w, cur.p);
     cur.blk = false;
     return cur.p >= l && cur.p < R;
+}
+
+// Arrays whose values stay in L2 beside their tables; a sector of a larger one
+// comes from DRAM.
+constexpr uint64_t kWarmN = uint64_t(1) << 24;
+
+// A query [l, R) shorter than the first window, in an array that stays in L2
+// (win_block reads those from DRAM by win_short_cover, whose few level-0
+// sectors are what counts there: lognormal(32, 0.7), n = 2^26, q = 2^25:
+// 698 us against 805).  The whole blocks inside it from V1, then the part of
+// the query in each of the two blocks at its ends from level 0, only where
+// that block's minimum is below (left: not above) theirs: 2.3 to 2.9 sectors
+// instead of 3.1 to 4.8 with both ends and no V1 minima to compare.  What
+// bounds it is the ALU pipe (70-75 % busy), so the lanes of a warp stay in
+// step (loads under a predicate, no branches around them) and the place of
+// the minimum is looked up once, at the end.  Length 24, n = 2^20, q = 2^22,
+// us: min + argmin 89 -> 75, minima 66 -> 52; lognormal(32, 0.7) 87 -> 82 and
+// 80 -> 68 (by blocks that touch the query, the failures listed and redone).
+// The last sector of level 0 must not be cut off (R <= n rounded down to 8).
+// SECTORS: of a block.  POS: the position is wanted.
+template <bool POS, uint32_t SECTORS, typename I>
+__device__ __forceinline__ WinBest<I> win_short(const WinViewT<I>& w, I l, I R) {
+    constexpr uint32_t blk = SECTORS == 1u ? 3u : 4u;
+    const I bl = l >> blk, br = (R - 1u) >> blk, b = bl & ~I(7);
+    const uint32_t i = uint32_t(bl - b), last = uint32_t(br - b);
+    WinBest<I> c{f_inf(), b, true};
+    float K[8], U[8];  // POS: the sector that holds c.v, its other entries masked out
+    ld_blocks8(w, b, K);
+    ld_blocks8_if(w, last > 7u, I(b + 8u), U);
+    const float vl = win_pick(K, i), v0 = win_pick(K, last & 7u), v1 = win_pick(U, last & 7u);
+    float vr = last < 8u ? v0 : v1;
+    const uint32_t hi = last < 16u ? last : 16u;
+    const uint32_t bits = ((1u << hi) - 1u) & ~((2u << i) - 1u);
+    const auto least = [](float (&v)[8], uint32_t mask) { return POS ? win_mask8(v, mask) : win_min8(v, mask); };
+    // x, the least of U, offered to c; `at`: U's first entry, of V1 or of level 0
+    const auto take = [&](float x, I at, bool block, bool ties) {
+        if (ties ? x <= c.v : x < c.v) {
+            c.v = x;
+            c.p = at;
+            c.blk = block;
+            if (POS) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) K[j] = U[j];
+            }
+        }
+    };
+    c.v = least(K, bits);
+    take(least(U, bits >> 8), I(b + 8u), true, false);
+#pragma unroll 1
+    for (uint32_t k = 16; k <= last; k += 8u) {
+        ld_blocks8(w, I(b + k), U);
+        vr = win_pick(U, last & 7u);
+        take(least(U, last - k < 8u ? (1u << (last - k)) - 1u : 255u), I(b + k), true, false);
+    }
+    const I e = (bl + 1u) << blk;
+    I lo = l, end = R < e ? R : e;
+    bool need = vl <= c.v;
+#pragma unroll 1
+    for (uint32_t side = 0; side < 2; ++side) {
+        const I s = lo & ~I(7);
+        const uint32_t part = need ? ((2u << uint32_t(end - 1u - s)) - 1u) & ~((1u << uint32_t(lo - s)) - 1u) : 0u;
+        if (SECTORS > 1u) {
+            float A[8];
+            ld_values8_if(w, need, s, A);
+            ld_values8_if(w, (part >> 8) != 0u, I(s + 8u), U);
+            float x = least(A, part);
+            const float y = least(U, part >> 8);
+            I at = s + 8u;
+            if (!(y < x)) {
+                at = s;
+                if (POS) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) U[j] = A[j];
+                }
+            } else {
+                x = y;
+            }
+            // as take(), which ptxas makes 6 % slower here
+            if (side ? x < c.v : x <= c.v) {
+                c.v = x;
+                c.p = at;
+                c.blk = false;
+                if (POS) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) K[j] = U[j];
+                }
+            }
+        } else {
+            ld_values8_if(w, need, s, U);
+            take(least(U, part), s, false, side == 0u);
+        }
+        lo = br << blk;
+        end = R;
+        need = vr < c.v;
+    }
+    if (POS) {
+        if (c.v < f_inf()) {
+            c.p += win_locate8(K, c.v);
+        } else {
+            c.p = l;
+            c.blk = false;
+        }
+    } else if (__float_as_uint(c.v) == 0x80000000u) {
+        // min.f32 takes -0 before +0: the sign is that of the query's first zero
+        I p = l;
+        while (w.a[p] != 0.0f) ++p;
+        c.v = w.a[p];
+    }
+    return c;
+}
+
+// A short query [l, R) in one round trip: its ends at level 0 and its whole
+// blocks, all read at once.  SECTORS: of a block.
+template <uint32_t SECTORS, typename I>
+__device__ __forceinline__ WinBest<I> win_short_once(const WinViewT<I>& w, I l, I R) {
+    const I bl = l >> w.blk, br = (R - 1u) >> w.blk;
+    const I a0 = l & ~I(7), ae = (bl + 1u) << w.blk, ar = R < ae ? R : ae;  // left end: [l, ar)
+    const I r0 = br << w.blk, b0 = (bl + 1u) & ~I(7);
+    const bool right = br != bl, a1 = SECTORS > 1u && a0 + 8u < ar,
+               r1 = SECTORS > 1u && right && r0 + 8u < R, mid = br > bl + 1u;
+    float A[8], A1[8], V[8], B[8], B1[8];
+    ld_values8(w, a0, A);
+    if (a1) ld_values8(w, I(a0 + 8u), A1);
+    if (right) ld_values8(w, r0, B);
+    if (r1) ld_values8(w, I(r0 + 8u), B1);
+    if (mid) ld_blocks8(w, b0, V);
+    const uint32_t abits = ((2u << uint32_t(ar - 1u - a0)) - 1u) & ~((1u << uint32_t(l - a0)) - 1u);
+    const uint32_t rbits = (2u << uint32_t(R - 1u - r0)) - 1u;
+    WinBest<I> c{f_inf(), l, false};
+    const auto take = [&](float (&u)[8], uint32_t bits, I s, bool blk) {
+        float x = win_mask8(u, bits);
+        if (x < c.v) {
+            c.p = s + win_locate8(u, x);
+            c.v = x;
+            c.blk = blk;
+        }
+    };
+    take(A, abits, a0, false);
+    if (a1) take(A1, abits >> 8, I(a0 + 8u), false);
+    if (mid) {
+        take(V, win_bits(uint32_t(bl + 1u - b0), br - b0 < 8u ? uint32_t(br - b0) : 8u), b0, true);
+#pragma unroll 1
+        for (I b = b0 + 8u; b < br; b += 8u) {
+            ld_blocks8(w, b, V);
+            take(V, win_bits(0u, br - b < 8u ? uint32_t(br - b) : 8u), b, true);
+        }
+    }
+    if (right) take(B, rbits, r0, false);
+    if (r1) take(B1, rbits >> 8, I(r0 + 8u), false);
+    return c;
 }
 
 // The exact answer of [l, R) from entries inside it, for a query whose cover
@@ -622,10 +815,10 @@ __device__ __forceinline__ I win_place(const WinViewT<I>& w, const WinBest<I>& c
 
 // Queries qs[0 .. cnt) (cnt <= sm.cap, a multiple of threads x LQ; every thread
 // of the block of `threads` calls), results to the same places of out_min /
-// out_idx (null: not wanted).
-// Returns this thread's number of invalid queries (l > r or r >= n), which
+// out_idx (null: not wanted).  COLD: level 0 is in DRAM (n > kWarmN).  ARGMIN:
+// of tables with argmin, whose blocks are of 16 entries.  Returns this thread's number of invalid queries (l > r or r >= n), which
 // get NaN and all ones.
-template <bool ARGMIN, uint32_t LQ, typename I>
+template <bool ARGMIN, bool COLD, uint32_t LQ, typename I>
 __device__ __forceinline__ uint32_t win_block(const WinViewT<I>& w, const WinLists<I>& sm, uint32_t threads,
                                               const typename IdxTraits<I>::Pair* __restrict__ qs, uint32_t cnt,
                                               float* __restrict__ out_min, I* __restrict__ out_idx) {
@@ -633,7 +826,7 @@ __device__ __forceinline__ uint32_t win_block(const WinViewT<I>& w, const WinLis
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t first = w.first;
     const bool tables = w.n >= (I(1) << first);
-    const I raw_limit = win_raw_limit<I>(w.n);
+    const I raw_limit = COLD ? win_raw_limit<I>(w.n) : I(16), whole = w.n & ~I(7);
     uint32_t bad = 0;
     const auto store = [&](const WinBest<I>& c, I l, uint32_t slot) {
         if (out_min != nullptr) st_stream(out_min + slot, c.v);
@@ -684,6 +877,10 @@ __device__ __forceinline__ uint32_t win_block(const WinViewT<I>& w, const WinLis
                 kind = 2u;
             } else if ((len >> (first - 1u)) == 0u || !tables) {
                 kind = 1u;
+                if (!COLD && r >= whole) {
+                    kind = 3u;
+                    bound[j] = f_nan();
+                }
             } else {
                 WinBest<I> c{__uint_as_float(e1[j].x), I(e1[j].y), false};
                 I p2 = I(e2[j].y);
@@ -697,7 +894,7 @@ __device__ __forceinline__ uint32_t win_block(const WinViewT<I>& w, const WinLis
                 if (covered && c.p >= l && c.p <= r) {
                     store(c, l, slot);
                 } else {
-                    kind = (len >> first) != 0u ? 3u : 1u;
+                    kind = (len >> first) != 0u || (!COLD && r >= whole) ? 3u : 1u;
                     bound[j] = covered ? c.v : f_nan();
                 }
             }
@@ -740,8 +937,6 @@ __device__ __forceinline__ uint32_t win_block(const WinViewT<I>& w, const WinLis
         }
     }
     __syncthreads();
-    // Short queries by their covering blocks (those that fail join the rest),
-    // the shortest at level 0.
     const uint32_t nshort = sm.count[0], nraw = sm.count[1];
 #pragma unroll 1
     for (uint32_t t0 = threadIdx.x - lane; t0 < nshort; t0 += threads) {
@@ -750,19 +945,27 @@ __device__ __forceinline__ uint32_t win_block(const WinViewT<I>& w, const WinLis
         if (t0 + lane < nshort) {
             slot = sm.first[t0 + lane];
             const Pair q = sm.q[slot];
+            const I l = q.x, R = q.y + 1u;
             WinBest<I> c;
-            fail = !win_short_cover(w, I(q.x), I(q.y + 1u), c);
-            if (!fail) store(c, I(q.x), slot);
+            if (COLD)
+                fail = !win_short_cover(w, l, R, c);
+            else if (ARGMIN || w.blk != 3u)
+                c = win_short<ARGMIN, 2>(w, l, R);
+            else
+                c = win_short<ARGMIN, 1>(w, l, R);
+            if (!fail) store(c, l, slot);
         }
-        const uint32_t mf = __ballot_sync(0xffffffffu, fail);
-        if (mf != 0u) {
-            uint32_t base = 0;
-            if (lane == 0u) base = atomicAdd(&sm.count[2], uint32_t(__popc(mf)));
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (fail) {
-                const uint32_t at = base + __popc(mf & ((1u << lane) - 1u));
-                sm.rest[at] = uint16_t(slot);
-                sm.bound[at] = f_nan();
+        if (COLD) {
+            const uint32_t mf = __ballot_sync(0xffffffffu, fail);
+            if (mf != 0u) {
+                uint32_t base = 0;
+                if (lane == 0u) base = atomicAdd(&sm.count[2], uint32_t(__popc(mf)));
+                base = __shfl_sync(0xffffffffu, base, 0);
+                if (fail) {
+                    const uint32_t at = base + __popc(mf & ((1u << lane) - 1u));
+                    sm.rest[at] = uint16_t(slot);
+                    sm.bound[at] = f_nan();
+                }
             }
         }
     }
@@ -772,7 +975,7 @@ __device__ __forceinline__ uint32_t win_block(const WinViewT<I>& w, const WinLis
         const Pair q = sm.q[slot];
         store(win_raw<3>(w, I(q.x), I(q.y + 1u)), I(q.x), slot);
     }
-    __syncthreads();
+    if (COLD) __syncthreads();
     const uint32_t nrest = sm.count[2];
 #pragma unroll 1
     for (uint32_t t = threadIdx.x; t < nrest; t += threads) {
@@ -786,47 +989,6 @@ __device__ __forceinline__ uint32_t win_block(const WinViewT<I>& w, const WinLis
         store(c, l, slot);
     }
     return bad;
-}
-
-// A short query [l, R) in one round trip: its ends at level 0 and its whole
-// blocks, all read at once.  SECTORS: of a block.
-template <uint32_t SECTORS, typename I>
-__device__ __forceinline__ WinBest<I> win_short_once(const WinViewT<I>& w, I l, I R) {
-    const I bl = l >> w.blk, br = (R - 1u) >> w.blk;
-    const I a0 = l & ~I(7), ae = (bl + 1u) << w.blk, ar = R < ae ? R : ae;  // left end: [l, ar)
-    const I r0 = br << w.blk, b0 = (bl + 1u) & ~I(7);
-    const bool right = br != bl, a1 = SECTORS > 1u && a0 + 8u < ar,
-               r1 = SECTORS > 1u && right && r0 + 8u < R, mid = br > bl + 1u;
-    float A[8], A1[8], V[8], B[8], B1[8];
-    ld_values8(w, a0, A);
-    if (a1) ld_values8(w, I(a0 + 8u), A1);
-    if (right) ld_values8(w, r0, B);
-    if (r1) ld_values8(w, I(r0 + 8u), B1);
-    if (mid) ld_blocks8(w, b0, V);
-    const uint32_t abits = ((2u << uint32_t(ar - 1u - a0)) - 1u) & ~((1u << uint32_t(l - a0)) - 1u);
-    const uint32_t rbits = (2u << uint32_t(R - 1u - r0)) - 1u;
-    WinBest<I> c{f_inf(), l, false};
-    const auto take = [&](float (&u)[8], uint32_t bits, I s, bool blk) {
-        float x = win_mask8(u, bits);
-        if (x < c.v) {
-            c.p = s + win_locate8(u, x);
-            c.v = x;
-            c.blk = blk;
-        }
-    };
-    take(A, abits, a0, false);
-    if (a1) take(A1, abits >> 8, I(a0 + 8u), false);
-    if (mid) {
-        take(V, win_bits(uint32_t(bl + 1u - b0), br - b0 < 8u ? uint32_t(br - b0) : 8u), b0, true);
-#pragma unroll 1
-        for (I b = b0 + 8u; b < br; b += 8u) {
-            ld_blocks8(w, b, V);
-            take(V, win_bits(0u, br - b < 8u ? uint32_t(br - b) : 8u), b, true);
-        }
-    }
-    if (right) take(B, rbits, r0, false);
-    if (r1) take(B1, rbits >> 8, I(r0 + 8u), false);
-    return c;
 }
 
 // One query [l, r] by one thread.

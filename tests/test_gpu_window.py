@@ -13,7 +13,7 @@ import rmq_gb300 as R
 pytestmark = pytest.mark.gpu
 
 SIZES = [1, 8, 9, 31, 33, 127, 128, 129, 255, 256, 257, 511, 513, 4097, 65_535, 65_536, 65_537,
-         (1 << 22) - 1, 1 << 22, (1 << 22) + 1, (1 << 22) + 65, 9_000_001]
+         (1 << 22) - 1, 1 << 22, (1 << 22) + 1, (1 << 22) + 65, 9_000_001, (1 << 24) + 13]
 KINDS = ["random", "ascending", "descending", "ties", "zeros", "inf"]
 LENGTHS = [1, 2, 7, 8, 9, 15, 16, 17, 31, 33, 63, 65, 127, 128, 129, 223, 224, 225, 255, 256, 257, 319, 321, 447, 449,
            511, 512, 513, 1023, 1025, 4095, 4097, 8191, 8193, 65_535, 65_537, 1 << 20, 1 << 22]
@@ -49,7 +49,7 @@ def test_window_tables_match_scan(cuda, n, kind):
     import torch
     rng = np.random.default_rng(n * 7 + KINDS.index(kind))
     dv = torch.from_numpy(_values(kind, n, rng)).to(cuda)
-    for q in (777, (1 << 17) + 5):  # below and above the few-queries kernel's limit
+    for q in (777, (1 << 18) + 5):  # below and above the few-queries kernel's limit
         qs = _queries(n, q, rng)
         if q == 777:
             qs[5] = (n - 1, 0) if n > 1 else (0, 1)  # invalid
@@ -69,3 +69,16 @@ def test_window_tables_match_scan(cuda, n, kind):
         assert torch.equal(i, bi)
         valid = bi != -1
         assert torch.equal(i64[valid], bi[valid].to(torch.int64)) and bool((i64[~valid] == -1).all())
+
+
+@pytest.mark.parametrize("n", [7, 40, 5000, 300_007])
+def test_positions_without_argmin_arrays(cuda, n):
+    """A handle without argmin arrays whose plan is level 0 alone (t >= n) still answers positions."""
+    import torch
+    rng = np.random.default_rng(n)
+    dv = torch.from_numpy(_values("ties", n, rng)).to(cuda)
+    for q in (777, (1 << 18) + 5):
+        dq = torch.from_numpy(_queries(n, q, rng).view(np.int32)).to(cuda)
+        _, bi = R.bruteforce(dv, dq)
+        with R.Hierarchy(dv, t=1 << 20, with_index=False) as h:
+            assert torch.equal(h.query_idx(dq), bi)
