@@ -32,8 +32,8 @@
 // Measured, min + argmin, against the block-minimum descent (one thread per
 // query, rf = 8) that it replaces, us per launch: lognormal(2^13, 1) lengths,
 // n = q = 2^26: 2567 -> 718; the mixture of three length laws with 1 % of the
-// values at the minimum, n = q = 2^26: 3377 -> 1617, n = 2^28, q = 2^27:
-// 9962 -> 4853; uniform lengths, minima, n = 5e7, q = 3e7: 1226 -> 240;
+// values at the minimum, n = q = 2^26: 3377 -> 1618, n = 2^28, q = 2^27:
+// 9962 -> 4801; uniform lengths, minima, n = 5e7, q = 3e7: 1226 -> 240;
 // lognormal(32, 0.7), positions, n = 2^26, q = 2^25: 1370 -> 698; 64-bit
 // positions, lognormal(2^13, 1), n = 2^26, q = 2^25: 1503 -> 567.
 #pragma once
@@ -670,7 +670,9 @@ __device__ __forceinline__ WinBest<I> win_short_once(const WinViewT<I>& w, I l, 
 // `bound` is a lower bound of the answer (the cover's minimum; NaN: none): an
 // entry equal to it that is found first from the left ends the search
 // (repeated minima: the usual case after a cover whose first occurrence lay
-// left of l).
+// left of l; in the first sector of V1 already for three in five where one
+// value in 100 is the minimum: the mixture of lengths with n = 2^28, q = 2^27
+// 4858 -> 4801 us).
 template <typename I>
 __device__ __forceinline__ void win_exact(const WinViewT<I>& w, I l, I R, float bound, WinBest<I>& cur, float& vl,
                                           float& vr) {
@@ -688,7 +690,7 @@ __device__ __forceinline__ void win_exact(const WinViewT<I>& w, I l, I R, float 
         vl = win_pick(v, uint32_t(bl - b));
         if (b == last && br != bl) vr = win_pick(v, uint32_t(br - b));
         win_take_blocks(v, win_bits(uint32_t(bl - b) + 1u, end <= b ? 0u : (end - b < 8u ? uint32_t(end - b) : 8u)), b, cur);
-        if (b == last) return;
+        if (b == last || cur.v == bound) return;
     }
     b += 8u;
     if (windows) {
