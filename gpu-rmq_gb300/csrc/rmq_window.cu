@@ -104,7 +104,8 @@ uint64_t window_bytes(uint64_t n, bool with_index) {
 // 2^18 queries, where it is the faster one only for short lengths but never
 // slower than the descent by more than a few percent.  Results in host memory
 // always come from it: its warps write whole 128-byte lines, which the
-// CPU-GPU link wants (2^22 queries, page-locked: 214 us against 385).
+// CPU-GPU link wants (2^22 queries, page-locked: 214 us against 385; n = q =
+// 2^26, results in page-locked memory: 2.78 ms against 5.26).
 //
 // kQueryThreads and the blocks per SM: the loads in flight live in the part
 // of the SM's 256 KiB that shared memory leaves (8 KiB per block here); with
@@ -152,10 +153,22 @@ win_one_kernel(WinViewT<I> w, const typename IdxTraits<I>::Pair* __restrict__ qs
     if (ARGMIN) st_stream(out_idx + i, win_place(w, c, l));
 }
 
+// Results outside device memory (page-locked host memory passed to a device
+// call)?  Asked only before launches that take several microseconds.
+static bool off_device(const void* p) {
+    if (p == nullptr) return false;
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeHost || at.type == cudaMemoryTypeUnregistered;
+}
+
 template <bool ARGMIN, typename I>
 static cudaError_t launch_window_typed(const QueryArgs& a, const WinViewT<I>& w,
                                        const typename IdxTraits<I>::Pair* qs, I* out_idx, cudaStream_t s) {
-    if (a.q <= kFewQueries || a.host_buffers)
+    if (a.q <= kFewQueries || a.host_buffers || off_device(a.out_min) || off_device(out_idx))
         return launch_with_window(win_one_kernel<ARGMIN, I>, uint32_t((a.q + kOneThreads - 1u) / kOneThreads), kOneThreads,
                                   a, s, w, qs, a.q, a.out_min, out_idx, a.err);
     return launch_with_window(w.n > kWarmN ? win_query_kernel<ARGMIN, true, I> : win_query_kernel<ARGMIN, false, I>,

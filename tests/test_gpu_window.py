@@ -82,3 +82,27 @@ def test_positions_without_argmin_arrays(cuda, n):
         _, bi = R.bruteforce(dv, dq)
         with R.Hierarchy(dv, t=1 << 20, with_index=False) as h:
             assert torch.equal(h.query_idx(dq), bi)
+
+
+def test_many_queries_into_page_locked_memory_and_captured(cuda):
+    """Above the few-queries limit: results in page-locked host memory through the device call, and a captured launch."""
+    import torch
+    n, q = 100_003, (1 << 18) + 77
+    rng = np.random.default_rng(3)
+    dv = torch.from_numpy(_values("random", n, rng)).to(cuda)
+    dq = torch.from_numpy(_queries(n, q, rng).view(np.int32)).to(cuda)
+    bm, bi = R.bruteforce(dv, dq)
+    with R.Hierarchy(dv) as h:
+        hi, hm = torch.empty(q, dtype=torch.int32).pin_memory(), torch.empty(q).pin_memory()
+        assert h.query_idx_raw(dq.data_ptr(), q, hi.data_ptr(), hm.data_ptr()) == R.RMQ_OK
+        torch.cuda.synchronize()
+        assert torch.equal(hi, bi.cpu()) and torch.equal(hm.view(torch.int32), bm.cpu().view(torch.int32))
+        di, dm = torch.zeros(q, dtype=torch.int32, device=cuda), torch.zeros(q, device=cuda)
+        s = torch.cuda.Stream()
+        s.wait_stream(torch.cuda.current_stream())
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            h.query_idx(dq, out_idx=di, out_min=dm, with_min=True)
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(di, bi) and torch.equal(dm.view(torch.int32), bm.view(torch.int32))
