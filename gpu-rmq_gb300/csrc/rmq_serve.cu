@@ -1,8 +1,8 @@
 // rmq_serve.cu — the range-minimum query server (include/rmq_gb300_serve.h).
 //
 // State: an arena (one cudaMalloc of the HBM budget, first-fit free list,
-// 256-byte granules) holding every resident array's values, coarse levels and
-// argmin arrays; a table of registered arrays (resident or evicted); a FIFO of
+// 256-byte granules) holding every resident array's values and window tables; a
+// table of registered arrays (resident or evicted); a FIFO of
 // pending requests; S slots, each a stream with pinned and device staging
 // for one batch.
 //
@@ -11,8 +11,8 @@
 // marks admitted arrays ready when their build event completes, and whenever
 // a slot is free packs the pending requests whose arrays are ready (FIFO, up
 // to max_batch_queries) into it and launches: one H2D of descriptors, work
-// units and queries, one query kernel (the batched per-warp kernel, one
-// descriptor per request), one D2H of the results, event.  Requests arriving while batches run are
+// units and queries, one query kernel (serve_query_kernel: a warp per 32
+// queries of one request), one D2H of the results, event.  Requests arriving while batches run are
 // admitted into the next free slot, so up to S batches overlap on the device
 // with builds of newly admitted arrays on their own stream.
 //
