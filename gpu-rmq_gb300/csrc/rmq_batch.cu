@@ -185,7 +185,7 @@ struct rmq_batch {
     uint32_t qblock = 128;  // threads per CTA of the query kernel (untuned default)
     int with_index = 1;
     int device = 0;
-    // tables
+    // tables, and after them the descriptors and lists below (one allocation)
     char* tables = nullptr;
     uint64_t lvl_capacity = 0;  // level entries of the deepest accepted plan (set_tuning's limit)
     uint64_t lvl_used = 0;      // level entries of the current plan
@@ -279,19 +279,39 @@ int lay_out(rmq_batch* b, cudaStream_t s) {
         const uint64_t tiles[4] = {t.block, t.low, t.mid, t.top};
         for (int i = 0; i < 4; ++i) off[i][a + 1] = off[i][a] + tiles[i];
     }
-    cudaError_t e = cudaMalloc(&b->tables, bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_descs, sizeof(ArrayDesc) * b->num_arrays);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(b->d_descs, b->h_descs.data(), sizeof(ArrayDesc) * b->num_arrays, cudaMemcpyHostToDevice, s);
-    for (int i = 0; i < 4 && e == cudaSuccess; ++i) {
+    // the tables, then the descriptors and the lists: one allocation, of some
+    // 50 us, and one release (create and destroy of 384 arrays: 341 us;
+    // the levels with an allocation each: 506)
+    uint64_t at = (bytes + 255u) & ~uint64_t(255);
+    const auto take = [&](uint64_t size) {
+        const uint64_t p = at;
+        at += (size + 255u) & ~uint64_t(255);
+        return p;
+    };
+    const uint64_t off_bytes = sizeof(uint64_t) * (b->num_arrays + 1), descs_at = take(sizeof(ArrayDesc) * b->num_arrays),
+                   q_off_at = take(off_bytes), blk_off_at = take(off_bytes);
+    uint64_t off_at[4] = {}, owner_at[4] = {};
+    for (int i = 0; i < 4; ++i) {
         TileWork& w = b->work[i];
         w.total = off[i][b->num_arrays];
         if (w.total == 0) continue;
+        off_at[i] = take(off_bytes);
+        owner_at[i] = take(sizeof(uint32_t) * w.total);
+    }
+    cudaError_t e = cudaMalloc(&b->tables, at);
+    if (e != cudaSuccess) return status_of(e);
+    for (const TileWork& w : b->work)
         if (w.total > 0x7FFFFFFFull) return RMQ_ERR_UNSUPPORTED;  // one CTA per tile
-        e = cudaMalloc(&w.d_off, sizeof(uint64_t) * (b->num_arrays + 1));
-        if (e == cudaSuccess) e = cudaMalloc(&w.d_owner, sizeof(uint32_t) * w.total);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(w.d_off, off[i].data(), sizeof(uint64_t) * (b->num_arrays + 1), cudaMemcpyHostToDevice, s);
+    b->d_descs = reinterpret_cast<ArrayDesc*>(b->tables + descs_at);
+    b->d_q_off = reinterpret_cast<uint64_t*>(b->tables + q_off_at);
+    b->d_blk_off = reinterpret_cast<uint64_t*>(b->tables + blk_off_at);
+    e = cudaMemcpyAsync(b->d_descs, b->h_descs.data(), sizeof(ArrayDesc) * b->num_arrays, cudaMemcpyHostToDevice, s);
+    for (int i = 0; i < 4 && e == cudaSuccess; ++i) {
+        TileWork& w = b->work[i];
+        if (w.total == 0) continue;
+        w.d_off = reinterpret_cast<uint64_t*>(b->tables + off_at[i]);
+        w.d_owner = reinterpret_cast<uint32_t*>(b->tables + owner_at[i]);
+        e = cudaMemcpyAsync(w.d_off, off[i].data(), off_bytes, cudaMemcpyHostToDevice, s);
         if (e == cudaSuccess) e = rmq::launch_fill_owner(w.d_off, b->num_arrays, w.d_owner, s);
     }
     const cudaError_t es = cudaStreamSynchronize(s);  // the host lists die here
@@ -408,8 +428,6 @@ int rmq_batch_create(const float* d_values, const uint64_t* value_offsets, const
     b->lvl_capacity = cap;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     cudaError_t e = cudaSuccess;
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_q_off, sizeof(uint64_t) * (num_arrays + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_blk_off, sizeof(uint64_t) * (num_arrays + 1));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->cap_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreate(&b->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&b->ev1);
@@ -648,13 +666,6 @@ void rmq_batch_destroy(rmq_batch* b) {
         if (b->ev0) cudaEventDestroy(b->ev0);
         if (b->ev1) cudaEventDestroy(b->ev1);
         cudaFree(b->tables);
-        cudaFree(b->d_descs);
-        for (TileWork& w : b->work) {
-            cudaFree(w.d_off);
-            cudaFree(w.d_owner);
-        }
-        cudaFree(b->d_q_off);
-        cudaFree(b->d_blk_off);
         cudaFree(b->d_owner);
         cudaGetLastError();
     }
