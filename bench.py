@@ -544,7 +544,8 @@ def plain_measure(n, q, lr, ties, t, seed, args, dev, stream, ws, *, tag_suffix=
         if not is_vl:
             roofline["l2"] = l2
     roofline["canonical_frac"] = canonical_bytes / (kernel_ms / 1e3) / 1e9 / peaks["hbm_gbs"]
-    build_bytes = 4 * n + 8 * sum(info.sizes()[1:])
+    # VL: the window tables with argmin take 1.0625 bytes per value
+    build_bytes = 4 * n + (17 * n // 16 if is_vl else 8 * sum(info.sizes()[1:]))
     rec = {"value": value, "unit": UNIT, "ms_per_step": total_ms / args.steps, "steps": args.steps,
            "warmup": args.warmup, "workload": workload_name(n, q, lr, ties),
            "n": n, "q": q, "lr_code": lr, "ties": ties, "seed": seed, "scan_threshold": t, "l2": l2_note,
