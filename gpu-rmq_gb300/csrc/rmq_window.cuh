@@ -49,9 +49,10 @@ namespace rmq {
 // levels with their stored indices take 1.143 and 0.571, so what fitted before
 // still fits, but for small arrays without argmin (2.3 MB more at 2^22).
 // Windows at every 16th of their size fail half as often as at every 8th,
-// which counts for more than short queries do: with blocks of eight entries and c = 3 for argmin too, 384 arrays of 2^10 .. 2^20 values
-// built and queried together take 2149 us instead of 1960, and n = 2^20, q =
-// 2^22, us, length 24: 65 instead of 75, lognormal(2^13, 1): 48 instead of 41.
+// which counts for more than short queries do: with blocks of eight entries
+// and c = 3 for argmin too, 384 arrays of 2^10 .. 2^20 values built and queried
+// together take 2149 us instead of 1960, and n = 2^20, q = 2^22, us, length 24:
+// 65 instead of 75, lognormal(2^13, 1): 48 instead of 41.
 // Without argmin blocks of eight pay for small arrays, whose short queries are
 // bound by instructions (length 24: 52 us, with blocks of 16: 67).
 struct WinForm {
