@@ -9,7 +9,7 @@
 // kernel one CTA per run of queries of one array.  Build + queries can be
 // captured as one CUDA graph.  384 arrays of 2^10 .. 2^20 values, 1.4e8
 // queries of lognormal(sqrt(size), 1) lengths, build and queries: 4125 us with
-// the block-minimum levels, 1960 us with the tables.
+// the block-minimum levels, 1949 us with the tables.
 #include <algorithm>
 #include <cstring>
 #include <new>
