@@ -75,9 +75,10 @@ constexpr uint64_t kVlT = 32;
 // AUTO resolves to VL: measured on GB300 it is the faster one at every batch
 // size and array size tried (n = q = 2^26: 93 G queries/s against 16.4).
 
-// Largest n of 32-bit handles: queries are uint32 pairs and the descent rounds
-// r up by at most rf - 1 without overflowing 32 bits.  64-bit handles take up
-// to 2^40 entries (4 TiB of values, far above any GPU's memory).
+// Largest n of 32-bit handles: queries are uint32 pairs, and what a query
+// rounds up (CL: r by at most rf - 1; the window tables: l by at most a
+// smallest stride, 2^8 entries) stays below 2^32.  64-bit handles take up to
+// 2^40 entries (4 TiB of values, far above any GPU's memory).
 constexpr uint64_t kMaxN = 0xFFFFFF00ull;
 constexpr uint64_t kMaxNWide = uint64_t(1) << 40;
 

@@ -219,8 +219,20 @@ __device__ __forceinline__ void win_load_view(const ArrayDesc& d, const float* v
     v.kmax = d.kmax;
 }
 
-__device__ __forceinline__ uint32_t win_log2(uint32_t x) { return 31u - uint32_t(__clz(int(x))); }
-__device__ __forceinline__ uint32_t win_log2(uint64_t x) { return 63u - uint32_t(__clzll((long long)x)); }
+__host__ __device__ __forceinline__ uint32_t win_log2(uint32_t x) {
+#ifdef __CUDA_ARCH__
+    return 31u - uint32_t(__clz(int(x)));
+#else
+    return 31u - uint32_t(__builtin_clz(x));
+#endif
+}
+__host__ __device__ __forceinline__ uint32_t win_log2(uint64_t x) {
+#ifdef __CUDA_ARCH__
+    return 63u - uint32_t(__clzll((long long)x));
+#else
+    return 63u - uint32_t(__builtin_clzll(x));
+#endif
+}
 
 // First entry of T_k.
 template <typename I, typename V>
@@ -660,6 +672,18 @@ __device__ __forceinline__ WinBest<I> win_short_once(const WinViewT<I>& w, I l, 
     return c;
 }
 
+// The part [x, y) of a query [l, R) that lies on whole strides of 2^gb: true
+// when it holds eight of them, so that windows inside the query serve it.
+// x does not wrap up to n = 0xFFFFFF00 (strides of at most 2^8); x plus eight
+// strides would, so the distance decides.
+template <typename I>
+__host__ __device__ __forceinline__ bool win_inner(I l, I R, uint32_t gb, I& x, I& y) {
+    const I gm = (I(1) << gb) - 1u;
+    x = (l + gm) & ~gm;
+    y = R & ~gm;
+    return y >= x && y - x >= (I(8) << gb);
+}
+
 // The exact answer of [l, R) from entries inside it, for a query whose cover
 // had its first minimum outside: all but the partial blocks at the two ends,
 // which are left to win_ends with their blocks' minima vl and vr (vr +inf: not
@@ -678,10 +702,9 @@ template <typename I>
 __device__ __forceinline__ void win_exact(const WinViewT<I>& w, I l, I R, float bound, WinBest<I>& cur, float& vl,
                                           float& vr) {
     const uint32_t gb = w.gb, step = w.c;
-    const I gm = (I(1) << gb) - 1u;
     const I bl = l >> w.blk, br = (R - 1u) >> w.blk, last = br & ~I(7);
-    I x = (l + gm) & ~gm, y = R & ~gm;
-    const bool windows = y >= x + (I(8) << gb);
+    I x, y;
+    const bool windows = win_inner(l, R, gb, x, y);
     const I by = y >> w.blk;
     I b = bl & ~I(7);
     {
@@ -804,7 +827,7 @@ __device__ __forceinline__ I win_raw_limit(I n) { return n > (I(1) << 27) ? I(8)
 // it lies: two windows of 2^k hold len + 2 strides - 2 entries when
 // len < 7/4 2^k (a stride is at most 1/8 of the window).
 template <typename I>
-__device__ __forceinline__ bool win_cover(const WinViewT<I>& w, I l, I r, I len, uint32_t& k, I& s1, I& s2) {
+__host__ __device__ __forceinline__ bool win_cover(const WinViewT<I>& w, I l, I r, I len, uint32_t& k, I& s1, I& s2) {
     k = win_log2(len);
     if ((len >> (k - 3u)) >= 14u) ++k;
     if (k < w.first) k = w.first;
