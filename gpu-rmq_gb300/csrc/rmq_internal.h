@@ -39,6 +39,9 @@ uint64_t tail_counters(const Layout& lay);
 uint64_t window_bytes(uint64_t n, bool with_index);
 cudaError_t launch_window_build(const float* d_values, void* tables, uint64_t n, bool with_index, bool wide,
                                 cudaStream_t s);
+// Loads the code of every kernel that a build with argmin and 32-bit
+// positions and its queries can launch, on the current device.
+cudaError_t load_window_kernels();
 
 struct QueryArgs {
     Levels lv;

@@ -9,14 +9,15 @@
 // The caller still provides the values, the queries and the output buffers.
 //
 // When the array exists on a device: CUDA loads device code lazily by default
-// (CUDA_MODULE_LOADING=LAZY), so the array, and the build and query kernels
-// this entry point launches, are placed on a device by the first call made
-// on it, not when the library is loaded.  That first call can therefore need
-// device memory for the array and the kernels' code; a caller that is about
-// to reserve the whole device should make one call (q = 0 is enough for the
-// array and the build kernel; q > 0 also loads the query kernel) before
-// reserving it, and before any stream capture.  From then on the device holds
-// the array until its context is destroyed (process exit or cudaDeviceReset).
+// (CUDA_MODULE_LOADING=LAZY), so the array is placed on a device by the first
+// call made on it, not when the library is loaded, and each kernel by whatever
+// names it first.  Which kernels a call launches depends on n and q, so the
+// first call on a device loads all of them, whatever its own n and q.  That
+// call can therefore need device memory for the array and the kernels' code; a
+// caller that is about to reserve the whole device should make one call (q = 0
+// is enough) before reserving it, and before any stream capture.  From then on
+// the device holds the array until its context is destroyed (process exit or
+// cudaDeviceReset).
 #include <cstring>
 #include <mutex>
 
@@ -91,6 +92,10 @@ int scratch_for_current_device(void** out) {
         void* p = nullptr;
         const cudaError_t e = cudaGetSymbolAddress(&p, g_scratch);
         if (e != cudaSuccess || p == nullptr) {
+            cudaGetLastError();
+            return RMQ_ERR_CUDA;
+        }
+        if (rmq::load_window_kernels() != cudaSuccess) {
             cudaGetLastError();
             return RMQ_ERR_CUDA;
         }

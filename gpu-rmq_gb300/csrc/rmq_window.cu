@@ -186,6 +186,24 @@ cudaError_t launch_window_query(const QueryArgs& a, cudaStream_t s) {
                                 : launch_window_typed<false, uint32_t>(a, a.win, a.qs, nullptr, s);
 }
 
+// The runtime loads a kernel's code with its first launch unless something
+// asks for its attributes before.
+cudaError_t load_window_kernels() {
+    const void* const kernels[] = {reinterpret_cast<const void*>(&win_block_kernel),
+                                   reinterpret_cast<const void*>(&win_low_kernel),
+                                   reinterpret_cast<const void*>(&win_mid_kernel),
+                                   reinterpret_cast<const void*>(&win_top_kernel),
+                                   reinterpret_cast<const void*>(&win_one_kernel<true, uint32_t>),
+                                   reinterpret_cast<const void*>(&win_query_kernel<true, false, uint32_t>),
+                                   reinterpret_cast<const void*>(&win_query_kernel<true, true, uint32_t>)};
+    for (const void* k : kernels) {
+        cudaFuncAttributes at;
+        const cudaError_t e = cudaFuncGetAttributes(&at, k);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
 #if RMQ_DEBUG_BOUNDS
 RMQ_BOUNDS_COUNTER_READER(bounds_bad_window)
 #endif

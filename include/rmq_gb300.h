@@ -174,18 +174,18 @@ const char* rmq_strerror(int status);
  * synchronise the device.  It has no counterpart in the reference.
  *
  * The window tables (t, the scan threshold, is checked as rmq_build checks
- * it; 0 = 32) are built into one fixed 8 MiB device array owned by the library, which every GPU that loads
- * the library holds until the process exits; then the queries are answered,
- * both on `stream`.  Limit: n <= 2^22 (4,194,304 entries); a larger n, or a t
- * whose levels do not fit, returns RMQ_ERR_UNSUPPORTED before any device
- * work.  The first call on each device (each device context: after a
- * cudaDeviceReset the next call counts as a first call again) looks up the
- * array's device address (cudaGetSymbolAddress).  CUDA loads device code
- * lazily by default, so that first call is also what places the array and
- * the kernels of this entry point on the device and may need device memory
- * for them: make it before reserving the whole device for a pool, and
- * before any stream capture (a call with q = 0 places the array and the
- * build kernel; one with q > 0 also the query kernel).
+ * it and has no other effect; 0 = 32) are built into one fixed 8 MiB device
+ * array owned by the library, which every GPU that loads the library holds
+ * until the process exits; then the queries are answered, both on `stream`.
+ * Limit: n <= 2^22 (4,194,304 entries); a larger n returns
+ * RMQ_ERR_UNSUPPORTED before any device work.  The first call on each device
+ * (each device context: after a cudaDeviceReset the next call counts as a
+ * first call again) looks up the array's device address
+ * (cudaGetSymbolAddress).  CUDA loads device code lazily by default, so that
+ * first call is also what places the array and every kernel of this entry
+ * point on the device, whatever its own n and q, and may need device memory
+ * for them: make it (q = 0 is enough) before reserving the whole device for a
+ * pool, and before any stream capture.
  * All calls on a device share the array, which keeps the last call's
  * contents (each call rewrites every entry it reads, so nothing needs
  * clearing): calls whose device work overlaps, on different streams or from
