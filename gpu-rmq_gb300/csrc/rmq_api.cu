@@ -628,10 +628,7 @@ int rmq_get_info(const rmq_handle* h, rmq_info* info) {
     if (h == nullptr || info == nullptr) return RMQ_ERR_ARG;
     fill_info(h->lay, h->variant, h->lanes, info);
     info->index_bits = h->wide ? 64 : 32;
-    // the levels of the plan; a VL handle's window tables take no more
-    info->level_bytes = h->lay.num_levels > 1
-                            ? h->lay.total * (sizeof(float) + (!h->with_index ? 0 : h->wide ? sizeof(uint64_t) : sizeof(uint32_t)))
-                            : 0;
+    info->level_bytes = h->level_bytes;
     info->build_ms = h->build_ms;
     return RMQ_OK;
 }

@@ -188,7 +188,7 @@ struct rmq_batch {
     // tables, and after them the descriptors and lists below (one allocation)
     char* tables = nullptr;
     uint64_t lvl_capacity = 0;  // level entries of the deepest accepted plan (set_tuning's limit)
-    uint64_t lvl_used = 0;      // level entries of the current plan
+    uint64_t table_bytes = 0;   // of all arrays
     uint32_t max_levels = 1;
     ArrayDesc* d_descs = nullptr;
     TileWork work[4];  // tiles of the block, low, mid and top kernels
@@ -260,7 +260,6 @@ int plan(rmq_batch* b, const uint64_t (&tc)[kClasses]) {
     for (int c = 0; c < kClasses; ++c) b->tc[c] = tc[c];
     b->t = tc[kClasses - 1];
     b->max_levels = max_levels;
-    b->lvl_used = base;
     return RMQ_OK;
 }
 
@@ -279,6 +278,7 @@ int lay_out(rmq_batch* b, cudaStream_t s) {
         const uint64_t tiles[4] = {t.block, t.low, t.mid, t.top};
         for (int i = 0; i < 4; ++i) off[i][a + 1] = off[i][a] + tiles[i];
     }
+    b->table_bytes = bytes;
     // the tables, then the descriptors and the lists: one allocation, of some
     // 50 us, and one release (create and destroy of 384 arrays: 341 us;
     // the levels with an allocation each: 506)
@@ -638,7 +638,7 @@ int rmq_batch_get_info(const rmq_batch* bc, rmq_batch_info* info) {
     std::memset(info, 0, sizeof(*info));
     info->num_arrays = b->num_arrays;
     for (uint64_t n : b->sizes) info->total_values += n;
-    info->level_bytes = b->lvl_used * (sizeof(float) + (b->with_index ? sizeof(uint32_t) : 0));
+    info->level_bytes = b->table_bytes;
     info->scan_threshold = b->t;
     info->query_block = b->qblock;
     info->max_levels = b->max_levels;

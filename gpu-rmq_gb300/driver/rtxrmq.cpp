@@ -546,7 +546,7 @@ void write_csv(const Args& a, const Result& r, const uint32_t* hQ, int check_cod
     // Column schema of create_XXX_header / create_header (src/tools.h:508-524);
     // this driver's columns follow checkResult.
     const char* extra = "variant,rf_log,lanes,event_qps,hbm_GBps,l2_GBps,roofline_frac,p50_us,p99_us,mode,"
-                        "hbm_peak_GBps\n";
+                        "hbm_peak_GBps,device_MB\n";
     if (!exists) {
         if (hier)
             std::fprintf(fp, "dev,alg,nt,reps,n,bs,nb,q,lr,GPU_BSIZE,CG_GROUP_SIZE,CG_MEM_ALIGNMENT,timestamp,"
@@ -591,11 +591,13 @@ void write_csv(const Args& a, const Result& r, const uint32_t* hQ, int check_cod
     else
         std::fprintf(fp, "%s,%s,%d,%d,%llu,1,0,%u,%d,%d,0,0,%s,", device, alg_name(a.alg), a.nt, a.reps,
                      (unsigned long long)a.n, a.q, a.lr, gpu_bsize, ts);
-    // outbuffer: the level buffer of block minima (MB), as the reference
-    // (src/xxx.h:269); tempbuffer: the stored argmin positions beside it.
+    // outbuffer: the planned levels' block minima (MB), as the reference
+    // (src/xxx.h:269); tempbuffer: their argmin positions.  CL holds both; what
+    // a handle really holds (VL: window tables) is in device_MB.
     const bool idx = is_idx_alg(a.alg);
-    const double lvl_mb = hier ? double(r.info.level_bytes) / 1e6 : 0.0;
-    const double out_mb = idx ? lvl_mb / 2 : lvl_mb, tmp_mb = idx ? lvl_mb / 2 : 0.0;
+    const uint32_t top = hier ? r.info.num_levels - 1 : 0;
+    const uint64_t entries = top > 0 ? (r.info.level_offset[top] + r.info.level_size[top] + 31) / 32 * 32 : 0;
+    const double out_mb = 4.0 * double(entries) / 1e6, tmp_mb = idx ? out_mb : 0.0;
     std::fprintf(fp, "%f,%f,%f,%f,%f,%f,%d,%f,%d,", r.total_ms / 1000.0, double(a.q) / (t_it / 1000.0),
                  t_it * 1e6 / a.q, double(r.build_ms), out_mb, tmp_mb, mem_ok, double(free_b) / 1048576.0,
                  check_code);
@@ -618,11 +620,12 @@ void write_csv(const Args& a, const Result& r, const uint32_t* hQ, int check_cod
             cudaGetLastError();
         }
         std::fprintf(fp, "%f,%f,", hbm, l2);
-        if (peak > 0) std::fprintf(fp, "%f,,,plain,%f\n", hbm / peak, peak);
-        else std::fprintf(fp, ",,,plain,\n");
+        if (peak > 0) std::fprintf(fp, "%f,,,plain,%f,", hbm / peak, peak);
+        else std::fprintf(fp, ",,,plain,,");
     } else {
-        std::fprintf(fp, ",,,,,%s,\n", is_gpu_alg(a.alg) ? "plain" : "cpu");
+        std::fprintf(fp, ",,,,,%s,,", is_gpu_alg(a.alg) ? "plain" : "cpu");
     }
+    std::fprintf(fp, "%f\n", r.out_mb);
     std::fclose(fp);
 }
 

@@ -76,6 +76,7 @@ typedef struct {
 } rmq_config;
 
 typedef struct {
+    /* the plan of levels by t and rf (num_levels, level_size, level_offset); CL handles hold it */
     uint32_t num_levels;        /* including level 0 (the caller's array)               */
     uint32_t rf_log;            /* reduction factor of every level step                 */
     int32_t  variant;           /* resolved variant (never AUTO)                         */
@@ -84,8 +85,8 @@ typedef struct {
     uint64_t scan_threshold;    /* resolved t                                            */
     uint64_t level_size[20];    /* entries per level                                     */
     uint64_t level_offset[20];  /* element offset of level k >= 1 in the level buffer    */
-    uint64_t level_bytes;       /* device bytes of level values (+ argmin arrays); a VL handle's window
-                                   tables take no more (n > 64)                           */
+    uint64_t level_bytes;       /* device bytes the handle holds: CL's level values (+ argmin arrays), VL's
+                                   window tables                                          */
     float    build_ms;          /* device time of the last build (CUDA events)           */
     int32_t  index_bits;        /* 32 or 64                                              */
 } rmq_info;

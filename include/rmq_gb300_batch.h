@@ -28,7 +28,7 @@ typedef struct rmq_batch rmq_batch;
 typedef struct {
     uint32_t num_arrays;
     uint64_t total_values;      /* sum of the array sizes                                   */
-    uint64_t level_bytes;       /* device bytes of all coarse levels (values + argmin)      */
+    uint64_t level_bytes;       /* device bytes of all arrays' window tables                */
     uint64_t scan_threshold;    /* t used for every array (after autotuning, if run)         */
     uint32_t query_block;       /* threads per CTA of the query kernel (one warp = 32 queries) */
     uint32_t max_levels;        /* deepest hierarchy in the batch                            */
