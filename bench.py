@@ -20,8 +20,7 @@ The default run adds `sub_records`, each with its own value, ms_per_step,
 roofline, parity sample and clocks:
   mixture_n2e26  n = q = 2^26, 1 % of entries tied at the minimum, lengths one
                  third each uniform [1, n], lognormal(2^13, 1), lognormal(2^5,
-                 0.7), t = 64 (the mixed-length target: the canonical
-                 descent's bytes at >= 0.60 of HBM peak)
+                 0.7), t = 64 (the mixed-length target: >= 0.60 of HBM peak)
   c3_n2e28       n = 2^28 with 1 % ties, q = 2^27, the same mixture, t = 64
   c1_n2e20       n = 2^20, q = 2^16, lengths uniform [1, n] (the reference's
                  CPU case), L2 flushed between steps, against the L2 read rate
@@ -506,8 +505,8 @@ def plain_measure(n, q, lr, ties, t, seed, args, dev, stream, ws, *, tag_suffix=
     peaks = measured_peaks()
     kernel_ms = statistics.mean(per_launch)
     # CL reads the canonical descent's level-0 sectors; the window tables of VL
-    # answer most queries without them, so VL counts what every method needs
-    # (the canonical figure stays beside it)
+    # answer most queries without them, so VL counts what every method needs.
+    # canonical_frac compares VL with CL and is no fraction of a roofline.
     canonical_bytes = algorithmic_bytes_chunked(qs, n)
     is_vl = info.variant in (2, 6)
     alg_bytes = needed_bytes(q, n, True, True) if is_vl else canonical_bytes
@@ -544,8 +543,7 @@ def plain_measure(n, q, lr, ties, t, seed, args, dev, stream, ws, *, tag_suffix=
         if not is_vl:
             roofline["l2"] = l2
     roofline["canonical_frac"] = canonical_bytes / (kernel_ms / 1e3) / 1e9 / peaks["hbm_gbs"]
-    # VL: the window tables with argmin take 1.0625 bytes per value
-    build_bytes = 4 * n + (17 * n // 16 if is_vl else 8 * sum(info.sizes()[1:]))
+    build_bytes = 4 * n + (int(info.level_bytes) if is_vl else 8 * sum(info.sizes()[1:]))
     rec = {"value": value, "unit": UNIT, "ms_per_step": total_ms / args.steps, "steps": args.steps,
            "warmup": args.warmup, "workload": workload_name(n, q, lr, ties),
            "n": n, "q": q, "lr_code": lr, "ties": ties, "seed": seed, "scan_threshold": t, "l2": l2_note,
@@ -574,8 +572,7 @@ def plain_measure(n, q, lr, ties, t, seed, args, dev, stream, ws, *, tag_suffix=
 PLAIN_SUBS = {
     "mixture_n2e26": {"n": 1 << 26, "q": 1 << 26, "lr": -8, "ties": 0.01, "t": 64, "tag": "-mixture",
                       "target": {"what": "plain kernel at n = 2^26 with mixed query lengths: "
-                                         "the canonical descent's bytes at >= 0.60 of the HBM peak",
-                                 "frac_at_least": 0.60}},
+                                         "roofline.frac >= 0.60 of the HBM peak", "frac_at_least": 0.60}},
     "c3_n2e28": {"n": 1 << 28, "q": 1 << 27, "lr": -8, "ties": 0.01, "t": 64, "tag": "-n2e28"},
     "c1_n2e20": {"n": 1 << 20, "q": 1 << 16, "lr": -1, "ties": 0.0, "t": 64, "tag": "-n2e20", "l2": True},
 }
@@ -677,7 +674,7 @@ def run_ours(args, ws, rank, local):
                 r, _ = plain_measure(c["n"], c["q"], c["lr"], c["ties"], c["t"], args.seed + rank, args, dev,
                                      stream, ws, tag_suffix=c["tag"], l2_bound=c.get("l2", False))
                 if "target" in c:
-                    r["target"] = dict(c["target"], met=bool(r["roofline"]["canonical_frac"] >= c["target"]["frac_at_least"]))
+                    r["target"] = dict(c["target"], met=bool(r["roofline"]["frac"] >= c["target"]["frac_at_least"]))
             elif name == "batched_c4":
                 r = batched_record(args, ws, rank, dev)
             else:
@@ -777,8 +774,8 @@ def targets_summary(subs: dict) -> dict:
     out = {}
     m = subs.get("mixture_n2e26", {})
     if "roofline" in m:
-        out["plain_mixture_n2e26_frac"] = {"value": m["roofline"]["canonical_frac"], "target": 0.60,
-                                          "met": m["roofline"]["canonical_frac"] >= 0.60}
+        out["plain_mixture_n2e26_frac"] = {"value": m["roofline"]["frac"], "target": 0.60,
+                                          "met": m["roofline"]["frac"] >= 0.60}
     b = subs.get("batched_c4", {})
     if "speedup_vs_plain_loop" in b:
         out["batched_vs_per_array_plain_loop"] = {"value": b["speedup_vs_plain_loop"], "target": 3.0,
