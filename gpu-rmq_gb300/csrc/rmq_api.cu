@@ -25,6 +25,7 @@ struct rmq_handle {
     uint32_t* idx_buf = nullptr;
     void* tables = nullptr;         // VL: the window tables
     unsigned* counters = nullptr;   // arrival counters of the single-launch build (after the levels)
+    uint32_t form = 0;              // of the window tables
     bool wide = false;
     uint32_t* err = nullptr;  // invalid-query counter (validate mode)
     int device = 0;
@@ -71,14 +72,14 @@ constexpr uint64_t kClT = 64;
 constexpr int kClLanes = 2;
 constexpr int kVlRfLog = 3;
 constexpr uint64_t kVlT = 32;
-// (VL: the plan that is reported; the window tables do not depend on it.)
+// (VL: the plan whose bytes its window tables keep to.)
 // AUTO resolves to VL: measured on GB300 it is the faster one at every batch
 // size and array size tried (n = q = 2^26: 93 G queries/s against 16.4).
 
 // Largest n of 32-bit handles: queries are uint32 pairs, and what a query
-// rounds up (CL: r by at most rf - 1; the window tables: l by at most a
-// smallest stride, 2^8 entries) stays below 2^32.  64-bit handles take up to
-// 2^40 entries (4 TiB of values, far above any GPU's memory).
+// rounds up (CL: r by at most rf - 1) stays below 2^32; where a window table's
+// strides do not, win_inner says so.  64-bit handles take up to 2^40 entries
+// (4 TiB of values, far above any GPU's memory).
 constexpr uint64_t kMaxN = 0xFFFFFF00ull;
 constexpr uint64_t kMaxNWide = uint64_t(1) << 40;
 
@@ -246,7 +247,9 @@ int rmq_build(const float* d_values, uint64_t n, const rmq_config* cfg, rmq_stre
     // (build, 2^20 queries and release of 20,000,003 values: 373 -> 271 us).
     size_t counter_bytes = 0;
     if (h->windows()) {
-        h->level_bytes = rmq::window_bytes(n, h->positions());
+        const uint64_t entry = sizeof(float) + (!h->with_index ? 0 : wide ? sizeof(uint64_t) : sizeof(uint32_t));
+        h->form = rmq::win_form_for(n, h->positions(), h->lay.num_levels > 1 ? h->lay.total * entry : 0);
+        h->level_bytes = rmq::win_shape(n, h->form).bytes;
     } else if (h->lay.num_levels > 1) {
         h->level_bytes = h->lay.total * (sizeof(float) + (h->with_index ? sizeof(uint32_t) : 0));
         counter_bytes = rmq::tail_counters(h->lay) * sizeof(unsigned);
@@ -277,7 +280,7 @@ int rmq_build(const float* d_values, uint64_t n, const rmq_config* cfg, rmq_stre
     if (e == cudaSuccess) e = cudaEventCreate(&e1);
     if (e == cudaSuccess) e = cudaEventRecord(e0, s);
     if (e == cudaSuccess)
-        e = h->windows() ? rmq::launch_window_build(d_values, h->tables, n, h->positions(), wide, s)
+        e = h->windows() ? rmq::launch_window_build(d_values, h->tables, n, h->form, wide, s)
                          : rmq::launch_build(h->lay, d_values, h->val_buf, h->idx_buf, s, h->counters);
     if (e == cudaSuccess) e = cudaEventRecord(e1, s);
     if (e == cudaSuccess) e = cudaEventSynchronize(e1);
@@ -318,8 +321,8 @@ static rmq::QueryArgs query_args(const rmq_handle* h, const void* d_lr, uint64_t
     rmq::QueryArgs a;
     std::memset(&a, 0, sizeof(a));
     if (h->windows()) {
-        if (h->wide) a.win64 = rmq::win_view<uint64_t>(h->d_values, h->tables, h->lay.n, h->positions());
-        else a.win = rmq::win_view<uint32_t>(h->d_values, h->tables, h->lay.n, h->positions());
+        if (h->wide) a.win64 = rmq::win_view<uint64_t>(h->d_values, h->tables, h->lay.n, h->form);
+        else a.win = rmq::win_view<uint32_t>(h->d_values, h->tables, h->lay.n, h->form);
     } else {
         for (uint32_t k = 0; k < h->lay.num_levels; ++k) {
             a.lv.val[k] = k == 0 ? h->d_values : h->val_buf + h->lay.offset[k];

@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(kBlockThreads)
 batch_block_kernel(const float* __restrict__ values, const ArrayDesc* __restrict__ descs, TileList l, char* tables) {
     WinOut w;
     const uint64_t tile = batch_tile(descs, l, values, tables, w);
-    win_block_tile(w, tile);
+    win_block_tile<false>(w, tile);
 }
 
 __global__ void __launch_bounds__(kLowThreads)
@@ -48,7 +48,7 @@ batch_low_kernel(const ArrayDesc* __restrict__ descs, TileList l, char* tables) 
     __shared__ uint2 sa[kSpan + kHaloLow], sb[kSpan + kHaloLow];
     WinOut w;
     const uint64_t tile = batch_tile(descs, l, nullptr, tables, w);
-    win_low_tile(w, tile, sa, sb);
+    win_low_tile<false>(w, tile, sa, sb);
 }
 
 __global__ void __launch_bounds__(kMidThreads)
@@ -95,7 +95,7 @@ batch_query_kernel(const float* __restrict__ values, const ArrayDesc* __restrict
     const WinLists<uint32_t> sm = win_lists<uint32_t>(batch_smem, cap);
     __syncthreads();
     // many arrays: each is small enough to count as warm, or rare
-    win_block<ARGMIN, false, kBatchLaneQueries>(view, sm, blockDim.x, qs + at, left < cap ? uint32_t(left) : cap,
+    win_block<ARGMIN, false, false, kBatchLaneQueries>(view, sm, blockDim.x, qs + at, left < cap ? uint32_t(left) : cap,
                                                 out_min != nullptr ? out_min + at : nullptr,
                                                 ARGMIN ? out_idx + at : nullptr);
 }
@@ -124,7 +124,7 @@ serve_query_kernel(const float* __restrict__ values, const ArrayDesc* __restrict
     const WinView& w = views[warp];
     const bool valid = in_range && Q.x <= Q.y && Q.y < w.n;
     WinBest<uint32_t> c{f_nan(), kNoPos, false};
-    if (valid) c = win_one(w, Q.x, Q.y);
+    if (valid) c = win_one<false>(w, Q.x, Q.y);
     if (in_range) {
         if (r.out_min != nullptr) st_stream(r.out_min + at, c.v);
         if (r.out_idx != nullptr) st_stream(r.out_idx + at, win_place(w, c, valid ? Q.x : kNoPos));
@@ -210,6 +210,9 @@ struct rmq_batch {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     bool build_timed = false;
     float build_ms = 0.f, query_ms = 0.f;
+
+    // Many arrays' tables take no more than levels did, so no blocks of eight.
+    uint32_t form() const { return with_index ? rmq::kFormArgmin : rmq::kFormMin; }
 };
 
 namespace {
@@ -271,7 +274,7 @@ int lay_out(rmq_batch* b, cudaStream_t s) {
     b->h_descs.resize(b->num_arrays);
     uint64_t bytes = 0;
     for (uint32_t a = 0; a < b->num_arrays; ++a) {
-        const rmq::WinShape w = rmq::win_shape(b->sizes[a], b->with_index != 0);
+        const rmq::WinShape w = rmq::win_shape(b->sizes[a], b->form());
         b->h_descs[a] = rmq::win_desc(b->val_off[a], bytes, w);
         bytes += w.bytes;
         const rmq::WinTiles t = rmq::win_tiles(w);
@@ -522,13 +525,13 @@ int rmq_batch_run_per_array(rmq_batch* b, rmq_stream_t stream) {
         const ArrayDesc& d = b->h_descs[a];
         const float* vals = b->d_values + d.val_off;
         char* tables = b->tables + d.win_off;
-        cudaError_t e = rmq::launch_window_build(vals, tables, b->sizes[a], b->with_index != 0, false, s);
+        cudaError_t e = rmq::launch_window_build(vals, tables, b->sizes[a], b->form(), false, s);
         if (e != cudaSuccess) return status_of(e);
         const uint64_t q0 = b->q_off[a], q = b->q_off[a + 1] - q0;
         if (q == 0) continue;
         rmq::QueryArgs qa;
         std::memset(&qa, 0, sizeof(qa));
-        qa.win = rmq::win_view<uint32_t>(vals, tables, b->sizes[a], b->with_index != 0);
+        qa.win = rmq::win_view<uint32_t>(vals, tables, b->sizes[a], b->form());
         qa.qs = reinterpret_cast<const uint2*>(b->d_lr) + q0;
         qa.q = q;
         qa.out_min = b->d_min != nullptr ? b->d_min + q0 : nullptr;

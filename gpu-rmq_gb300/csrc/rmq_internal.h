@@ -34,12 +34,11 @@ cudaError_t launch_build(const Layout& lay, const float* d_values, float* val_bu
 // Arrival counters the single-launch build needs for `lay` (0: none).
 uint64_t tail_counters(const Layout& lay);
 
-// Window tables (rmq_window.cuh) of n values into `tables` (window_bytes
+// Window tables (rmq_window.cuh) of n values into `tables` (the shape's
 // bytes, 32-byte aligned).
-uint64_t window_bytes(uint64_t n, bool with_index);
-cudaError_t launch_window_build(const float* d_values, void* tables, uint64_t n, bool with_index, bool wide,
+cudaError_t launch_window_build(const float* d_values, void* tables, uint64_t n, uint32_t form, bool wide,
                                 cudaStream_t s);
-// Loads the code of every kernel that a build with argmin and 32-bit
+// Loads the code of every kernel that a build of kFormArgmin with 32-bit
 // positions and its queries can launch, on the current device.
 cudaError_t load_window_kernels();
 
@@ -70,7 +69,6 @@ cudaError_t launch_window_query(const QueryArgs& a, cudaStream_t s);
 
 cudaError_t launch_bruteforce(const float* vals, uint32_t n, const uint2* qs, uint32_t q,
                               float* out_min, uint32_t* out_idx, cudaStream_t s);
-
 // Queries per work unit: threads x kBatchLaneQueries of a batched CTA, and of
 // a warp of the served kernel.
 constexpr uint32_t kBatchLaneQueries = 4;

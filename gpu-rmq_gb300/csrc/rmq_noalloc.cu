@@ -121,7 +121,7 @@ extern "C" int rmq_query_idx_static(const float* d_values, uint64_t n, uint64_t 
     if (n > kStaticMaxN || q > 0xFFFFFFFFull) return RMQ_ERR_UNSUPPORTED;  // above the fixed scratch
     const uint64_t t = scan_threshold != 0 ? scan_threshold : kStaticDefaultT;
     if (t < (uint64_t(1) << kStaticRfLog)) return RMQ_ERR_ARG;  // VL precondition, src/xxx.h:938
-    if (rmq::window_bytes(n, true) > kScratchBytes) return RMQ_ERR_UNSUPPORTED;
+    if (rmq::win_shape(n, rmq::kFormArgmin).bytes > kScratchBytes) return RMQ_ERR_UNSUPPORTED;
 
     void* scratch = nullptr;
     const int st = scratch_for_current_device(&scratch);
@@ -130,11 +130,11 @@ extern "C" int rmq_query_idx_static(const float* d_values, uint64_t n, uint64_t 
 
     // Every table entry a query reads is rewritten by the build of this call, so nothing
     // in the scratch needs clearing between calls.
-    cudaError_t e = rmq::launch_window_build(d_values, scratch, n, true, false, s);
+    cudaError_t e = rmq::launch_window_build(d_values, scratch, n, rmq::kFormArgmin, false, s);
     if (e == cudaSuccess && q > 0) {
         rmq::QueryArgs a;
         std::memset(&a, 0, sizeof(a));
-        a.win = rmq::win_view<uint32_t>(d_values, scratch, n, true);
+        a.win = rmq::win_view<uint32_t>(d_values, scratch, n, rmq::kFormArgmin);
         a.qs = reinterpret_cast<const uint2*>(d_lr);
         a.q = q;
         a.out_min = d_min_or_null;

@@ -51,6 +51,7 @@ struct ServedArray {
     uint64_t n = 0, seed = 0;
     const float* host = nullptr;
     uint64_t bytes = 0, val_bytes = 0;
+    uint32_t form = 0;  // of its window tables
     bool resident = false, ready = false, admitted_before = false;
     uint64_t off = 0;  // arena byte offset
     int pins = 0;
@@ -151,7 +152,7 @@ struct rmq_server {
 namespace {
 
 rmq::ArrayDesc describe(const ServedArray& a) {
-    return rmq::win_desc(a.off / 4, a.off + a.val_bytes, rmq::win_shape(a.n, true));
+    return rmq::win_desc(a.off / 4, a.off + a.val_bytes, rmq::win_shape(a.n, a.form));
 }
 
 void evict(rmq_server* s, uint64_t id) {
@@ -186,7 +187,7 @@ bool admit(rmq_server* s, uint64_t id) {
     } else {
         st = rmq_gen_values_device(vals, a.n, a.seed, reinterpret_cast<rmq_stream_t>(s->build_stream));
     }
-    if (st == RMQ_OK && rmq::launch_window_build(vals, s->arena + a.off + a.val_bytes, a.n, true, false, s->build_stream) != cudaSuccess) st = RMQ_ERR_CUDA;
+    if (st == RMQ_OK && rmq::launch_window_build(vals, s->arena + a.off + a.val_bytes, a.n, a.form, false, s->build_stream) != cudaSuccess) st = RMQ_ERR_CUDA;
     if (st == RMQ_OK && cudaEventRecord(a.built, s->build_stream) != cudaSuccess) st = RMQ_ERR_CUDA;
     if (st != RMQ_OK) {
         cudaGetLastError();
@@ -431,6 +432,18 @@ void dispatcher_main(rmq_server* s) {
     }
 }
 
+// The finest form of blocks of 16 entries (serve_query_kernel's) that takes no
+// more of the arena than the levels of scan threshold t at rf = 8, values and
+// positions each in granules of their own; the coarsest of them where none does
+// (arrays of up to t entries, which have no levels).
+uint32_t served_form(uint64_t n, uint64_t t) {
+    const rmq::Layout lay = rmq::plan_layout(n, t, 3);
+    const uint64_t levels = lay.num_levels > 1 ? 2 * rmq::arena_round_up(lay.total * sizeof(float)) : 0;
+    for (uint32_t f : {rmq::kFormArgmin, rmq::kFormMin})
+        if (rmq::arena_round_up(rmq::win_shape(n, f).bytes) <= levels) return f;
+    return rmq::kFormMin + 1;
+}
+
 int register_array(rmq_server* s, uint64_t n, uint64_t seed, const float* host, uint64_t* id) {
     if (s == nullptr || id == nullptr || n == 0) return RMQ_ERR_ARG;
     if (n > 0xFFFFFF00ull) return RMQ_ERR_UNSUPPORTED;
@@ -439,7 +452,8 @@ int register_array(rmq_server* s, uint64_t n, uint64_t seed, const float* host, 
     a.seed = seed;
     a.host = host;
     a.val_bytes = rmq::arena_round_up(n * sizeof(float));
-    a.bytes = a.val_bytes + rmq::arena_round_up(rmq::window_bytes(n, true));
+    a.form = served_form(n, s->cfg.scan_threshold);
+    a.bytes = a.val_bytes + rmq::arena_round_up(rmq::win_shape(n, a.form).bytes);
     if (a.bytes > s->cfg.hbm_budget_bytes) return RMQ_ERR_OOM;
     if (cudaEventCreateWithFlags(&a.built, cudaEventDisableTiming) != cudaSuccess) return RMQ_ERR_CUDA;
     std::lock_guard<std::mutex> lock(s->mu);

@@ -12,16 +12,18 @@ namespace rmq {
 __device__ __forceinline__ void wait_previous_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void allow_next_grid() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+template <bool LARGE>
 __global__ void __launch_bounds__(kBlockThreads) win_block_kernel(WinOut w) {
     allow_next_grid();
-    win_block_tile(w, blockIdx.x);
+    win_block_tile<LARGE>(w, blockIdx.x);
 }
 
+template <bool EIGHT>
 __global__ void __launch_bounds__(kLowThreads) win_low_kernel(WinOut w) {
     __shared__ uint2 sa[kSpan + kHaloLow], sb[kSpan + kHaloLow];
     wait_previous_grid();
     allow_next_grid();
-    win_low_tile(w, blockIdx.x, sa, sb);
+    win_low_tile<EIGHT>(w, blockIdx.x, sa, sb);
 }
 
 __global__ void __launch_bounds__(kMidThreads) win_mid_kernel(WinOut w) {
@@ -54,9 +56,9 @@ static cudaError_t launch_dependent(void (*kernel)(KArgs...), uint32_t grid, uin
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-cudaError_t launch_window_build(const float* d_values, void* tables, uint64_t n, bool with_index, bool wide,
+cudaError_t launch_window_build(const float* d_values, void* tables, uint64_t n, uint32_t form, bool wide,
                                 cudaStream_t s) {
-    const WinShape sh = win_shape(n, with_index);
+    const WinShape sh = win_shape(n, form);
     WinOut w;
     char* b = static_cast<char*>(tables);
     w.a = d_values;
@@ -73,16 +75,13 @@ cudaError_t launch_window_build(const float* d_values, void* tables, uint64_t n,
     w.kmax = sh.kmax;
     w.wide = wide;
     const WinTiles t = win_tiles(sh);
-    win_block_kernel<<<uint32_t(t.block), kBlockThreads, 0, s>>>(w);
+    (sh.blk > 4u ? win_block_kernel<true> : win_block_kernel<false>)<<<uint32_t(t.block), kBlockThreads, 0, s>>>(w);
     cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess && t.low > 0) e = launch_dependent(win_low_kernel, uint32_t(t.low), kLowThreads, s, w);
+    if (e == cudaSuccess && t.low > 0) e = launch_dependent(sh.gb - sh.blk == 3u ? win_low_kernel<true> : win_low_kernel<false>,
+                                                        uint32_t(t.low), kLowThreads, s, w);
     if (e == cudaSuccess && t.mid > 0) e = launch_dependent(win_mid_kernel, uint32_t(t.mid), kMidThreads, s, w);
     if (e == cudaSuccess && t.top > 0) e = launch_dependent(win_top_kernel, uint32_t(t.top), kMidThreads, s, w);
     return e;
-}
-
-uint64_t window_bytes(uint64_t n, bool with_index) {
-    return win_shape(n, with_index).bytes;
 }
 
 // ---------------------------------------------------------------------------
@@ -119,7 +118,7 @@ constexpr uint32_t kBlockQueries = kQueryThreads * kLaneQueries;
 constexpr uint32_t kOneThreads = 64;
 constexpr uint64_t kFewQueries = uint64_t(1) << 18;
 
-template <bool ARGMIN, bool COLD, typename I>
+template <bool ARGMIN, bool COLD, typename I, bool LARGE = false>
 __global__ void __launch_bounds__(kQueryThreads, sizeof(I) == 4 ? (ARGMIN ? 9 : 10) : 8)
 win_query_kernel(WinViewT<I> w, const typename IdxTraits<I>::Pair* __restrict__ qs, uint64_t q,
                  float* __restrict__ out_min, I* __restrict__ out_idx, uint32_t* __restrict__ err) {
@@ -127,13 +126,13 @@ win_query_kernel(WinViewT<I> w, const typename IdxTraits<I>::Pair* __restrict__ 
     const uint64_t at = uint64_t(blockIdx.x) * kBlockQueries;
     const uint32_t cnt = q - at < kBlockQueries ? uint32_t(q - at) : kBlockQueries;
     const WinLists<I> sm = win_lists<I>(smem, kBlockQueries);
-    const uint32_t bad = win_block<ARGMIN, COLD, kLaneQueries>(w, sm, kQueryThreads, qs + at, cnt,
+    const uint32_t bad = win_block<ARGMIN, COLD, LARGE, kLaneQueries>(w, sm, kQueryThreads, qs + at, cnt,
                                                                out_min != nullptr ? out_min + at : nullptr,
                                                                ARGMIN ? out_idx + at : nullptr);
     if (bad != 0u && err != nullptr) atomicAdd(err, bad);
 }
 
-template <bool ARGMIN, typename I>
+template <bool ARGMIN, typename I, bool LARGE = false>
 __global__ void __launch_bounds__(kOneThreads)
 win_one_kernel(WinViewT<I> w, const typename IdxTraits<I>::Pair* __restrict__ qs, uint64_t q,
                float* __restrict__ out_min, I* __restrict__ out_idx, uint32_t* __restrict__ err) {
@@ -145,7 +144,7 @@ win_one_kernel(WinViewT<I> w, const typename IdxTraits<I>::Pair* __restrict__ qs
     I l = IdxTraits<I>::none;
     if (Q.x <= Q.y && Q.y < w.n) {
         l = Q.x;
-        c = win_one(w, l, I(Q.y));
+        c = win_one<LARGE>(w, l, I(Q.y));
     } else if (err != nullptr) {
         atomicAdd(err, 1u);
     }
@@ -168,10 +167,14 @@ static bool off_device(const void* p) {
 template <bool ARGMIN, typename I>
 static cudaError_t launch_window_typed(const QueryArgs& a, const WinViewT<I>& w,
                                        const typename IdxTraits<I>::Pair* qs, I* out_idx, cudaStream_t s) {
+    const bool large = w.blk > 4u;
     if (a.q <= kFewQueries || a.host_buffers || off_device(a.out_min) || off_device(out_idx))
-        return launch_with_window(win_one_kernel<ARGMIN, I>, uint32_t((a.q + kOneThreads - 1u) / kOneThreads), kOneThreads,
-                                  a, s, w, qs, a.q, a.out_min, out_idx, a.err);
-    return launch_with_window(w.n > kWarmN ? win_query_kernel<ARGMIN, true, I> : win_query_kernel<ARGMIN, false, I>,
+        return launch_with_window(large ? win_one_kernel<ARGMIN, I, true> : win_one_kernel<ARGMIN, I>,
+                                  uint32_t((a.q + kOneThreads - 1u) / kOneThreads), kOneThreads, a, s, w, qs, a.q,
+                                  a.out_min, out_idx, a.err);
+    return launch_with_window(large             ? win_query_kernel<ARGMIN, true, I, true>
+                              : w.n > kWarmN    ? win_query_kernel<ARGMIN, true, I>
+                                                : win_query_kernel<ARGMIN, false, I>,
                               uint32_t((a.q + kBlockQueries - 1u) / kBlockQueries), kQueryThreads, a, s, w, qs, a.q,
                               a.out_min, out_idx, a.err);
 }
@@ -189,8 +192,8 @@ cudaError_t launch_window_query(const QueryArgs& a, cudaStream_t s) {
 // The runtime loads a kernel's code with its first launch unless something
 // asks for its attributes before.
 cudaError_t load_window_kernels() {
-    const void* const kernels[] = {reinterpret_cast<const void*>(&win_block_kernel),
-                                   reinterpret_cast<const void*>(&win_low_kernel),
+    const void* const kernels[] = {reinterpret_cast<const void*>(&win_block_kernel<false>),
+                                   reinterpret_cast<const void*>(&win_low_kernel<false>),
                                    reinterpret_cast<const void*>(&win_mid_kernel),
                                    reinterpret_cast<const void*>(&win_top_kernel),
                                    reinterpret_cast<const void*>(&win_one_kernel<true, uint32_t>),

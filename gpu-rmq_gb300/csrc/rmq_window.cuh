@@ -44,25 +44,46 @@ namespace rmq {
 
 // Sizes of the tables: log2 of the block, of the smallest stride, of the
 // strides per window (from window 2^(gb + c) on; smaller ones keep the
-// smallest stride), and of the first window.  Bytes per value: 1.0625 with
-// argmin, without 0.5625, and 1.125 up to 2^22 entries; the block-minimum
-// levels with their stored indices take 1.143 and 0.571, so what fitted before
-// still fits, but for small arrays without argmin (2.3 MB more at 2^22).
-// Windows at every 16th of their size fail half as often as at every 8th,
-// which counts for more than short queries do: with blocks of eight entries
-// and c = 3 for argmin too, 384 arrays of 2^10 .. 2^20 values built and queried
-// together take 2149 us instead of 1960, and n = 2^20, q = 2^22, us, length 24:
-// 65 instead of 75, lognormal(2^13, 1): 48 instead of 41.
-// Without argmin blocks of eight pay for small arrays, whose short queries are
-// bound by instructions (length 24: 52 us, with blocks of 16: 67).
+// smallest stride), and of the first window.
 struct WinForm {
     uint32_t blk, gb, c, first;
 };
+
+// The forms, with their bytes per value.  A handle takes the finest one that
+// needs no more than the levels that its scan threshold t and reduction factor
+// rf plan (win_form_for): a caller chooses its memory by those.  With argmin (8
+// bytes per level entry, 12 with 64-bit positions) levels take 1.143 bytes per
+// value at rf = 8, 0.533 at 16 and 0.258 at 32; without, half of the 8-byte
+// figures; a little less for a large t, nothing for t >= n, where the last form
+// is taken all the same.  The coarser forms lose on short and middle lengths.
+// n = 2^26, q = 2^24, min + argmin, us, at rf 8 / 16 / 32, and what descending
+// such levels took:
+//   lognormal(32, 0.7)    365 / 351 / 486     707 / 752 / 850
+//   length 500            171 / 469 / 385     677 / 715 / 844
+//   lognormal(2^13, 1)    184 / 224 / 248     655 / 854 / 1092
+//   uniform lengths       135 / 150 / 150     758 / 1150 / 1376
+// Only minima of lengths up to about 60 in arrays that stay in L2 were faster
+// there (n = 2^23, rf = 16, length 24: 267 us, here 297).
+//
+// Windows at every 16th of their size (kFormArgmin) fail half as often as at
+// every 8th, which counts for more than short queries do: with blocks of eight
+// entries and c = 3 for argmin too, 384 arrays of 2^10 .. 2^20 values built and
+// queried together take 2149 us instead of 1960, and n = 2^20, q = 2^22, us,
+// length 24: 65 instead of 75, lognormal(2^13, 1): 48 instead of 41.
+// Up to kSmallN entries the levels do not count: argmin tables take 4.3 MiB at
+// most, and without argmin blocks of eight (4.5 MiB at most, 2.3 MB more than
+// levels at rf = 8) pay, since short queries are bound by instructions there
+// (length 24: 52 us, with blocks of 16: 67).
+constexpr WinForm kForms[] = {
+    {4, 5, 4, 8},   // 1.0625
+    {3, 5, 3, 8},   // 1.125
+    {4, 6, 3, 9},   // 0.5625
+    {4, 7, 3, 10},  // 0.4375
+    {5, 8, 3, 11},  // 0.2188
+    {6, 9, 3, 12},  // 0.1094
+};
+constexpr uint32_t kFormArgmin = 0, kFormSmallMin = 1, kFormMin = 2, kFormLast = 5;
 constexpr uint64_t kSmallN = uint64_t(1) << 22;
-__host__ __device__ inline WinForm win_form(uint64_t n, bool with_index) {
-    if (with_index) return WinForm{4, 5, 4, 8};
-    return n <= kSmallN ? WinForm{3, 5, 3, 8} : WinForm{4, 6, 3, 9};
-}
 constexpr uint32_t kMaxWinLog = 32;  // largest window (offsets are 32-bit)
 
 // log2 of the stride of windows of 2^k entries.
@@ -98,8 +119,8 @@ struct WinShape {
     uint32_t blk, gb, c, first, kmax;
 };
 
-__host__ __device__ inline WinShape win_shape(uint64_t n, bool with_index) {
-    const WinForm f = win_form(n, with_index);
+inline WinShape win_shape(uint64_t n, uint32_t form) {
+    const WinForm f = kForms[form];
     WinShape w;
     w.n = n;
     w.blk = f.blk;
@@ -125,6 +146,14 @@ __host__ __device__ inline WinShape win_shape(uint64_t n, bool with_index) {
     return w;
 }
 
+// The form of an array's tables: `levels`, the bytes that its planned levels take.
+inline uint32_t win_form_for(uint64_t n, bool with_index, uint64_t levels) {
+    if (n <= kSmallN) return with_index ? kFormArgmin : kFormSmallMin;
+    uint32_t f = with_index ? kFormArgmin : kFormMin;
+    while (f < kFormLast && win_shape(n, f).bytes > levels) f = f < kFormMin ? kFormMin : f + 1u;
+    return f;
+}
+
 // The tables as the kernels see them (I: position type).
 template <typename I>
 struct WinViewT {
@@ -139,8 +168,8 @@ using WinView = WinViewT<uint32_t>;
 using WinView64 = WinViewT<uint64_t>;
 
 template <typename I>
-inline WinViewT<I> win_view(const float* a, const void* base, uint64_t n, bool with_index) {
-    const WinShape w = win_shape(n, with_index);
+inline WinViewT<I> win_view(const float* a, const void* base, uint64_t n, uint32_t form) {
+    const WinShape w = win_shape(n, form);
     WinViewT<I> v;
     const char* b = static_cast<const char*>(base);
     v.a = a;
@@ -448,6 +477,20 @@ __device__ __forceinline__ WinBest<I> win_raw(const WinViewT<I>& w, I lo, I hi) 
     return c;
 }
 
+// The same over any number of sectors, two at a time (four at once spill).
+template <typename I>
+__device__ __forceinline__ WinBest<I> win_raw_long(const WinViewT<I>& w, I lo, I hi) {
+    WinBest<I> c{f_inf(), lo, false};
+#pragma unroll 1
+    for (I at = lo; at < hi;) {
+        const I cut = (at & ~I(15)) + 16u, end = hi < cut ? hi : cut;
+        const WinBest<I> d = win_raw<2>(w, at, end);
+        if (d.v < c.v) c = d;
+        at = end;
+    }
+    return c;
+}
+
 // The blocks b + j, j in the bits of `mask`, of a loaded sector, offered to cur.
 template <typename I>
 __device__ __forceinline__ void win_take_blocks(float (&v)[8], uint32_t mask, I b, WinBest<I>& cur) {
@@ -494,8 +537,8 @@ __device__ __forceinline__ void win_blocks(const WinViewT<I>& w, I b0, I b1, Win
 // cur's position (it wins ties), the right one after.  vl, vr: the whole
 // blocks' minima; +inf leaves the right end out.  A block's stored first
 // minimum serves when it lies inside the query; otherwise its part of the
-// query is read at level 0.
-template <typename I>
+// query is read at level 0.  LARGE: blocks of more than 16 entries.
+template <bool LARGE, typename I>
 __device__ __forceinline__ void win_ends(const WinViewT<I>& w, I l, I R, float vl, float vr, WinBest<I>& cur) {
 #pragma unroll 1
     for (uint32_t side = 0; side < 2; ++side) {
@@ -505,7 +548,7 @@ __device__ __forceinline__ void win_ends(const WinViewT<I>& w, I l, I R, float v
         const I s = b << w.blk, p = s + ld_block_off(w, b);
         const I e = s + (I(1) << w.blk), lo = s < l ? l : s, hi = e < R ? e : R;
         WinBest<I> c{vb, p, false};
-        if (p < lo || p >= hi) c = win_raw<2>(w, lo, hi);
+        if (p < lo || p >= hi) c = LARGE ? win_raw_long(w, lo, hi) : win_raw<2>(w, lo, hi);
         if (side ? c.v < cur.v : c.v <= cur.v) cur = c;
     }
 }
@@ -674,14 +717,15 @@ __device__ __forceinline__ WinBest<I> win_short_once(const WinViewT<I>& w, I l, 
 
 // The part [x, y) of a query [l, R) that lies on whole strides of 2^gb: true
 // when it holds eight of them, so that windows inside the query serve it.
-// x does not wrap up to n = 0xFFFFFF00 (strides of at most 2^8); x plus eight
-// strides would, so the distance decides.
+// Within eight strides of 2^32 sums with x wrap, and x itself within one of
+// 2^9, so the distance decides: y - x is no more than the query's length just
+// where neither x nor the difference has wrapped.
 template <typename I>
 __host__ __device__ __forceinline__ bool win_inner(I l, I R, uint32_t gb, I& x, I& y) {
     const I gm = (I(1) << gb) - 1u;
     x = (l + gm) & ~gm;
     y = R & ~gm;
-    return y >= x && y - x >= (I(8) << gb);
+    return y - x <= R - l && y - x >= (I(8) << gb);
 }
 
 // The exact answer of [l, R) from entries inside it, for a query whose cover
@@ -817,9 +861,11 @@ __device__ __forceinline__ WinLists<I> win_lists(unsigned char* smem, uint32_t c
 // them (n = 2^20, q = 2^22, length 8 / 16: 49 / 62 us against 103 / 98).
 // Beyond 2^27 entries only up to eight: there the address translation of
 // random level-0 sectors bounds the chip at 55 G sectors/s (n = 2^28, length
-// 16: 231 us at level 0, 158 by blocks).
-template <typename I>
-__device__ __forceinline__ I win_raw_limit(I n) { return n > (I(1) << 27) ? I(8) : I(16); }
+// 16: 231 us at level 0, 158 by blocks).  LARGE: up to 32 entries, since a
+// cover of blocks of 32 or 64 fails for most of them (n = 2^23, q = 2^24,
+// blocks of 32, length 24: 354 us against 480; length 40: 455 against 439).
+template <bool LARGE, typename I>
+__device__ __forceinline__ I win_raw_limit(I n) { return n > (I(1) << 27) ? I(8) : I(LARGE ? 32 : 16); }
 
 // The two windows of T_k that cover [l, r] (len entries, at least half the
 // first window): starts s1 <= s2, equal when one window covers it.  k is the
@@ -849,9 +895,10 @@ __device__ __forceinline__ I win_place(const WinViewT<I>& w, const WinBest<I>& c
 // Queries qs[0 .. cnt) (cnt <= sm.cap, a multiple of threads x LQ; every thread
 // of the block of `threads` calls), results to the same places of out_min /
 // out_idx (null: not wanted).  COLD: level 0 is in DRAM (n > kWarmN).  ARGMIN:
-// of tables with argmin, whose blocks are of 16 entries.  Returns this thread's number of invalid queries (l > r or r >= n), which
-// get NaN and all ones.
-template <bool ARGMIN, bool COLD, uint32_t LQ, typename I>
+// of tables with positions, whose blocks are not of eight entries.  LARGE: blocks
+// of more than 16 entries (COLD only).  Returns this thread's number of invalid
+// queries (l > r or r >= n), which get NaN and all ones.
+template <bool ARGMIN, bool COLD, bool LARGE, uint32_t LQ, typename I>
 __device__ __forceinline__ uint32_t win_block(const WinViewT<I>& w, const WinLists<I>& sm, uint32_t threads,
                                               const typename IdxTraits<I>::Pair* __restrict__ qs, uint32_t cnt,
                                               float* __restrict__ out_min, I* __restrict__ out_idx) {
@@ -859,7 +906,7 @@ __device__ __forceinline__ uint32_t win_block(const WinViewT<I>& w, const WinLis
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t first = w.first;
     const bool tables = w.n >= (I(1) << first);
-    const I raw_limit = COLD ? win_raw_limit<I>(w.n) : I(16), whole = w.n & ~I(7);
+    const I raw_limit = COLD ? win_raw_limit<LARGE, I>(w.n) : I(16), whole = w.n & ~I(7);
     uint32_t bad = 0;
     const auto store = [&](const WinBest<I>& c, I l, uint32_t slot) {
         if (out_min != nullptr) st_stream(out_min + slot, c.v);
@@ -1006,7 +1053,8 @@ __device__ __forceinline__ uint32_t win_block(const WinViewT<I>& w, const WinLis
     for (uint32_t t = threadIdx.x; t < nraw; t += threads) {
         const uint32_t slot = sm.first[sm.cap - 1u - t];
         const Pair q = sm.q[slot];
-        store(win_raw<3>(w, I(q.x), I(q.y + 1u)), I(q.x), slot);
+        const I l = q.x, R = q.y + 1u;
+        store(LARGE ? win_raw_long(w, l, R) : win_raw<3>(w, l, R), l, slot);
     }
     if (COLD) __syncthreads();
     const uint32_t nrest = sm.count[2];
@@ -1018,14 +1066,15 @@ __device__ __forceinline__ uint32_t win_block(const WinViewT<I>& w, const WinLis
         WinBest<I> c = win_none<I>();
         float vl = f_inf(), vr = f_inf();
         win_exact(w, l, R, sm.bound[t], c, vl, vr);
-        win_ends(w, l, R, vl, vr, c);
+        win_ends<LARGE>(w, l, R, vl, vr, c);
         store(c, l, slot);
     }
     return bad;
 }
 
-// One query [l, r] by one thread.
-template <typename I>
+// One query [l, r] by one thread.  LARGE: blocks of more than 16 entries, whose
+// short queries go by win_exact as well.
+template <bool LARGE, typename I>
 __device__ __forceinline__ WinBest<I> win_one(const WinViewT<I>& w, I l, I r) {
     const I R = r + 1u, len = R - l;
     float bound = f_nan();
@@ -1039,11 +1088,11 @@ __device__ __forceinline__ WinBest<I> win_one(const WinViewT<I>& w, I l, I r) {
         if (covered && c.p >= l && c.p <= r) return c;
         if (covered) bound = c.v;
     }
-    if ((len >> w.first) == 0u) return w.blk == 3u ? win_short_once<1>(w, l, R) : win_short_once<2>(w, l, R);
+    if (!LARGE && (len >> w.first) == 0u) return w.blk == 3u ? win_short_once<1>(w, l, R) : win_short_once<2>(w, l, R);
     WinBest<I> c = win_none<I>();
     float vl = f_inf(), vr = f_inf();
     win_exact(w, l, R, bound, c, vl, vr);
-    win_ends(w, l, R, vl, vr, c);
+    win_ends<LARGE>(w, l, R, vl, vr, c);
     return c;
 }
 

@@ -2,7 +2,7 @@
 // the single-array kernels (rmq_window.cu) and the batched ones (rmq_batch.cu).
 //
 // One streaming pass over level 0 writes the minimum and its offset for every
-// block of 16 entries (0.31 n bytes); everything above is computed from those,
+// block (0.31 n bytes with blocks of 16 entries); everything above is computed from those,
 // which are still in L2.  A tile pass holds 2048 strides and a halo of 512 in
 // shared memory and makes every table whose windows fit the halo; a second
 // tile pass does the same for the next six sizes; one CTA makes the few
@@ -34,7 +34,9 @@ __host__ __device__ __forceinline__ uint32_t win_mid_log(const V& w) { return w.
 // Blocks of one tile.  A warp's load covers 32 consecutive sectors (1 KiB);
 // each lane takes its sector's first minimum, and the two lanes of a block
 // exchange one sector each of two loads, so that every lane ends with one
-// whole block and a warp stores 32 consecutive blocks.
+// whole block and a warp stores 32 consecutive blocks.  LARGE: blocks of 32 or
+// 64 entries, four or eight lanes each.
+template <bool LARGE>
 __device__ __forceinline__ void win_block_tile(const WinOut& w, uint64_t tile) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint64_t base = tile * kBlockTile;
@@ -73,6 +75,27 @@ __device__ __forceinline__ void win_block_tile(const WinOut& w, uint64_t tile) {
         }
         m[i] = mv;
         off[i] = j;
+    }
+    if (LARGE) {
+        const uint32_t sectors = 1u << (w.blk - 3u);
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) {
+            off[i] += 8u * (lane & (sectors - 1u));
+            for (uint32_t o = 1; o < sectors; o <<= 1) {
+                const float ov = __shfl_down_sync(0xffffffffu, m[i], o);
+                const uint32_t oo = __shfl_down_sync(0xffffffffu, off[i], o);
+                if (ov < m[i]) {  // the first lane of each 2 o: equal, its entry stays
+                    m[i] = ov;
+                    off[i] = oo;
+                }
+            }
+            const uint64_t sec = sec0 + 32u * i;
+            if ((lane & (sectors - 1u)) == 0u && (sec << 3) < w.n) {
+                w.v1[sec >> (w.blk - 3u)] = m[i];
+                w.j1[sec >> (w.blk - 3u)] = uint8_t(off[i]);
+            }
+        }
+        return;
     }
     if (w.blk == 3u) {  // a sector is a block
 #pragma unroll
@@ -139,14 +162,28 @@ __device__ __forceinline__ void win_double_up(const WinOut& w, uint32_t k, uint3
     }
 }
 
-// First minimum of the blocks of stride g (g < S), as an entry of T.
+// First minimum of the blocks of stride g (g < S), as an entry of T.  EIGHT: a
+// stride is eight blocks, else two or four.
+template <bool EIGHT>
 __device__ __forceinline__ uint2 win_group(const WinOut& w, uint64_t g) {
-    const uint32_t bpg = 1u << (w.gb - w.blk);  // blocks per stride: 2 or 4
+    constexpr uint32_t kMost = EIGHT ? 8u : 4u;
+    const uint32_t bpg = EIGHT ? 8u : 1u << (w.gb - w.blk);
     const uint64_t nb = (w.n + (uint64_t(1) << w.blk) - 1) >> w.blk, b = g * bpg;
-    float v[4];
-    uint32_t off;
+    float v[kMost];
+    uint64_t off;
     // V1 and J1 are padded to 32 bytes, so a whole stride of either can be read
-    if (bpg == 2u) {
+    if (EIGHT) {
+        const float4 x = *reinterpret_cast<const float4*>(w.v1 + b), y = *reinterpret_cast<const float4*>(w.v1 + b + 4);
+        v[0] = x.x;
+        v[1] = x.y;
+        v[2] = x.z;
+        v[3] = x.w;
+        v[kMost - 4] = y.x;
+        v[kMost - 3] = y.y;
+        v[kMost - 2] = y.z;
+        v[kMost - 1] = y.w;
+        off = *reinterpret_cast<const uint64_t*>(w.j1 + b);
+    } else if (bpg == 2u) {
         const float2 x = *reinterpret_cast<const float2*>(w.v1 + b);
         v[0] = x.x;
         v[1] = x.y;
@@ -160,10 +197,11 @@ __device__ __forceinline__ uint2 win_group(const WinOut& w, uint64_t g) {
         v[3] = x.w;
         off = *reinterpret_cast<const uint32_t*>(w.j1 + b);
     }
-    uint2 e = make_uint2(__float_as_uint(v[0]), off & 255u);
+    uint2 e = make_uint2(__float_as_uint(v[0]), uint32_t(off) & 255u);
 #pragma unroll
-    for (uint32_t c = 1; c < 4; ++c)
-        if (c < bpg && b + c < nb) e = win_first(e, make_uint2(__float_as_uint(v[c]), (off >> (8u * c)) & 255u), c << w.blk);
+    for (uint32_t c = 1; c < kMost; ++c)
+        if (c < bpg && b + c < nb)
+            e = win_first(e, make_uint2(__float_as_uint(v[c]), uint32_t(off >> (8u * c)) & 255u), c << w.blk);
     if (!w.wide) e.y += uint32_t(b << w.blk);
     return e;
 }
@@ -174,6 +212,7 @@ __device__ __forceinline__ uint2 win_group(const WinOut& w, uint64_t g) {
 // every thread keeps its entries in registers, all loads of a step in flight
 // (one tile: 16 -> 8.5 us against one entry after another with 256 threads;
 // the build of 2^20 values 25 -> 19 us, of 2^26 80 -> 71 us).
+template <bool EIGHT>
 __device__ __forceinline__ void win_low_tile(const WinOut& w, uint64_t tile, uint2* sa, uint2* sb) {
     constexpr uint32_t kPer = (kSpan + kHaloLow) / kLowThreads;
     const uint64_t g0 = tile * kSpan;
@@ -181,7 +220,7 @@ __device__ __forceinline__ void win_low_tile(const WinOut& w, uint64_t tile, uin
 #pragma unroll
     for (uint32_t u = 0; u < kPer; ++u) {
         const uint64_t g = g0 + threadIdx.x + kLowThreads * u;
-        if (g < w.S) e[u] = win_group(w, g);
+        if (g < w.S) e[u] = win_group<EIGHT>(w, g);
     }
     // Windows of 2, 4, 8 strides (2^first entries), the last one the first
     // table; where the next one has the same stride, a doubling of 8.

@@ -63,8 +63,12 @@ typedef enum {
 } rmq_variant;
 
 typedef struct {
-    /* t and rf plan the levels that CL handles hold and rmq_get_info reports;
-     * a VL handle checks and reports them, its window tables do not depend on them. */
+    /* t and rf plan the levels that CL handles hold and rmq_get_info reports.
+     * A VL handle's window tables take no more than those levels (4 bytes per
+     * entry, with argmin 8, or 12 with 64-bit positions) would: a larger rf or
+     * t makes them coarser.  Except: up to 2^22 values they take what serves
+     * queries best (at most 1.125 bytes per value), and where t >= n plans no
+     * levels, 0.11 bytes per value. */
     int32_t  variant;         /* rmq_variant                                                    */
     uint64_t scan_threshold;  /* t: build levels while a level holds more than t entries (0 = variant default) */
     int32_t  rf_log;          /* log2 of the per-level reduction factor, 3..5 (0 = variant default)       */

@@ -21,11 +21,13 @@ extern "C" {
 typedef struct rmq_server rmq_server;
 
 typedef struct {
-    uint64_t hbm_budget_bytes;    /* device arena for values + levels (default 64 GiB)           */
+    uint64_t hbm_budget_bytes;    /* device arena for values + tables (default 64 GiB)           */
     uint32_t slots;               /* batches in flight at once, each on its own stream (default 4) */
     uint64_t max_batch_queries;   /* queries per batch launch (default 2^21; >= 2^16)             */
     uint32_t max_batch_requests;  /* requests per batch (default 4096)                            */
-    uint64_t scan_threshold;      /* t of every served array (default 64)                         */
+    uint64_t scan_threshold;      /* t (default 64, >= 8): an array's window tables take no more of the arena than
+                                     the levels that t plans at rf = 8 would; an array of up to t values, which has
+                                     none, takes up to 0.44 bytes per value + 512 for them   */
     uint32_t query_threads;       /* CTA size of the query kernel (default 256)                   */
 } rmq_server_config;
 

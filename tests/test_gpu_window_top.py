@@ -44,8 +44,8 @@ def test_last_entries_of_32_bit_handles(cuda, n):
     local = _local(n - t0, Q, rng)
     bm, bi = R.bruteforce(v[t0:], _pairs(local, cuda))
     dq = _pairs(local + t0, cuda)
-    for with_index in (True, False):
-        with R.Hierarchy(v, with_index=with_index, index_bits=32) as h:
+    for with_index, rf_log in ((True, 3), (False, 3), (True, 5), (False, 5)):
+        with R.Hierarchy(v, with_index=with_index, rf_log=rf_log, index_bits=32) as h:
             m = h.query(dq)
             assert torch.equal(_bits(m), _bits(bm))
             if with_index:

@@ -25,8 +25,8 @@ def harness(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("with_index", [0, 1])
-def test_positions_near_2_pow_32(harness, with_index):
-    out = subprocess.run([str(harness), str(with_index)], capture_output=True, text=True, check=True).stdout
+@pytest.mark.parametrize("form", range(6))
+def test_positions_near_2_pow_32(harness, form):
+    out = subprocess.run([str(harness), str(form)], capture_output=True, text=True, check=True).stdout
     checked, wrong = out.split()[-3], out.split()[-1]
     assert int(checked) > 8_000_000 and wrong == "0", out
