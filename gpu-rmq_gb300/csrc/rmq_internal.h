@@ -69,6 +69,10 @@ cudaError_t launch_window_query(const QueryArgs& a, cudaStream_t s);
 
 cudaError_t launch_bruteforce(const float* vals, uint32_t n, const uint2* qs, uint32_t q,
                               float* out_min, uint32_t* out_idx, cudaStream_t s);
+// Results outside device memory (page-locked host memory passed to a device
+// call)?  Null: no.
+bool off_device(const void* p);
+
 // Queries per work unit: threads x kBatchLaneQueries of a batched CTA, and of
 // a warp of the served kernel.
 constexpr uint32_t kBatchLaneQueries = 4;

@@ -152,9 +152,8 @@ win_one_kernel(WinViewT<I> w, const typename IdxTraits<I>::Pair* __restrict__ qs
     if (ARGMIN) st_stream(out_idx + i, win_place(w, c, l));
 }
 
-// Results outside device memory (page-locked host memory passed to a device
-// call)?  Asked only before launches that take several microseconds.
-static bool off_device(const void* p) {
+// Asked only before launches that take several microseconds.
+bool off_device(const void* p) {
     if (p == nullptr) return false;
     cudaPointerAttributes at;
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {

@@ -53,7 +53,8 @@ int rmq_batch_create(const float* d_values, const uint64_t* value_offsets, const
  * d_lr[2i], d_lr[2i+1] for query_offsets[a] <= i < query_offsets[a+1]
  * (host array of num_arrays + 1 non-decreasing offsets; indices local to
  * array a).  Results go to the same positions of d_argmin (may be NULL for
- * minima only) and d_min (may be NULL when d_argmin is given).  Uploads the
+ * minima only) and d_min (may be NULL when d_argmin is given); either may lie in
+ * page-locked host memory, which takes a kernel of its own.  Uploads the
  * work list (synchronises `stream`); invalidates a captured graph. */
 int rmq_batch_set_queries(rmq_batch* b, const uint32_t* d_lr, const uint64_t* query_offsets,
                           uint32_t* d_argmin, float* d_min, rmq_stream_t stream);
