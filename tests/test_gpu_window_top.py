@@ -1,6 +1,7 @@
 """Window tables at the largest sizes (GPU): 32-bit handles up to 0xFFFFFF00
-entries, whose positions end just below 2^32; always more queries than the
-few-queries kernel takes."""
+entries, whose positions end just below 2^32, and 64-bit handles beyond 2^33,
+where a query can be longer than the two largest windows; always more queries
+than the few-queries kernel takes."""
 from __future__ import annotations
 
 import numpy as np
@@ -74,3 +75,32 @@ def test_long_queries_of_the_largest_32_bit_handle(cuda):
     for k in list(range(4)) + list(rng.integers(0, Q, 12)):
         lo, hi = int(lr[k, 0]), int(lr[k, 1])
         assert int(i64[k]) == lo + int(torch.argmin(v[lo:hi + 1]))
+
+
+def test_64_bit_handle_past_2_pow_33_entries(cuda):
+    """n = 2^33 + 2^25 + 8: queries across 2^32 equal a 32-bit handle's on that
+    part, and queries longer than two windows of 2^32 equal torch's scan, with
+    and without argmin tables."""
+    import torch
+    n = (1 << 33) + (1 << 25) + 8
+    rng = np.random.default_rng(6)
+    v = torch.empty(n, dtype=torch.float32, device=cuda)
+    R.gen_values_device(v, 79)
+    w0, wn = (1 << 32) - (1 << 25), 1 << 26
+    local = _local(wn, Q, rng)
+    long = np.array([(0, n - 1), (1, n - 1), (12_345, n - 6), (3, (1 << 33) + 900), ((1 << 25) - 9, n - 1),
+                     ((1 << 32) - 5, (1 << 32) + 5), (7, (1 << 32) + 1000), (1 << 31, n - 77)], dtype=np.int64)
+    many = np.tile(long, (Q // len(long) + 1, 1))
+    expect = torch.tensor([int(a) + int(torch.argmin(v[int(a):int(b) + 1])) for a, b in long], device=cuda)
+    for with_index, rf_log in ((True, 3), (False, 3), (True, 5)):
+        with R.Hierarchy(v, with_index=with_index, rf_log=rf_log) as h, R.Hierarchy(v[w0:w0 + wn]) as part:
+            pi, pm = part.query_idx(_pairs(local, cuda), with_min=True)
+            at = expect.repeat(Q // len(long) + 1)
+            if with_index:
+                i, m = h.query_idx64(_pairs(local + w0, cuda, np.int64), with_min=True)
+                assert torch.equal(i, pi.to(torch.int64) + w0)
+                j, k = h.query_idx64(_pairs(many, cuda, np.int64), with_min=True)
+                assert torch.equal(j, at)
+            else:
+                m, k = h.query64(_pairs(local + w0, cuda, np.int64)), h.query64(_pairs(many, cuda, np.int64))
+            assert torch.equal(_bits(m), _bits(pm)) and torch.equal(_bits(k), _bits(v[at]))
