@@ -219,7 +219,7 @@ struct rmq_batch {
     int device = 0;
     // tables, and after them the descriptors and lists below (one allocation)
     char* tables = nullptr;
-    uint64_t lvl_capacity = 0;  // level entries of the deepest accepted plan (set_tuning's limit)
+    uint64_t lvl_capacity = 0;  // entries of the deepest plan that set_tuning accepts (nothing is built of a plan)
     uint64_t table_bytes = 0;   // of all arrays
     uint32_t max_levels = 1;
     ArrayDesc* d_descs = nullptr;
@@ -453,7 +453,7 @@ int rmq_batch_create(const float* d_values, const uint64_t* value_offsets, const
     b->val_off.assign(value_offsets, value_offsets + num_arrays);
     b->sizes.assign(sizes, sizes + num_arrays);
     b->with_index = cfg != nullptr ? (cfg->with_index != 0) : 1;
-    // capacity: the deepest layout among the user's t and the tuner's candidates
+    // the deepest layout among the user's t and the tuner's candidates
     uint64_t cap = 0;
     for (uint32_t a = 0; a < num_arrays; ++a) {
         uint64_t m = layout_entries(sizes[a], t);

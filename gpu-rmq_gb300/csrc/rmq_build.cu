@@ -28,7 +28,7 @@ __device__ __forceinline__ void wait_previous_grid() { asm volatile("griddepcont
 // wait_previous_grid until this grid completes).
 __device__ __forceinline__ void allow_next_grid() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// One output block per group of LPB = rf/8 lanes .
+// One output block per group of LPB = rf/8 lanes.
 //   src, src_size : level k (level 0 = caller's array, not padded)
 //   src_idx       : level-0 indices of level k's entries (null for k = 0)
 //   src_padded    : src has at least round_up(src_size, 8) readable entries
@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(256)
 build_step_kernel(const float* __restrict__ src, const uint32_t* __restrict__ src_idx, uint32_t src_size, int src_padded,
                   float* __restrict__ dst, uint32_t* __restrict__ dst_idx, uint32_t dst_size) {
     constexpr uint32_t LPB = (1u << R) / 8u;
-        wait_previous_grid();
+    wait_previous_grid();
     allow_next_grid();
     const uint64_t gt = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     const uint32_t blk = uint32_t(gt / LPB);

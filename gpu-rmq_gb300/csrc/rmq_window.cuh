@@ -581,7 +581,10 @@ constexpr uint64_t kWarmN = uint64_t(1) << 24;
 // the minimum is looked up once, at the end.  Length 24, n = 2^20, q = 2^22,
 // us: min + argmin 89 -> 75, minima 66 -> 52; lognormal(32, 0.7) 87 -> 82 and
 // 80 -> 68 (by blocks that touch the query, the failures listed and redone).
-// The last sector of level 0 must not be cut off (R <= n rounded down to 8).
+// The query must be longer than a block, so that its ends lie in two blocks (with
+// both in one, the right end's part would begin before l): callers answer up to
+// 16 entries by win_raw.  The last sector of level 0 must not be cut off
+// (R <= n rounded down to 8).
 // SECTORS: of a block.  POS: the position is wanted.
 template <bool POS, uint32_t SECTORS, typename I>
 __device__ __forceinline__ WinBest<I> win_short(const WinViewT<I>& w, I l, I R) {

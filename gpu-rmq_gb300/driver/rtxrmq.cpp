@@ -118,10 +118,11 @@ void print_help() {
                  "  --data-dir <dir>        where those files go (default .)\n"
                  "  --log_build_threshold[=<k>]  accepted for command-line compatibility (no effect here)\n"
                  "  --save-power[=<file>]   accepted for command-line compatibility (power is not measured)\n"
-                 "  --variant <name>        work distribution of alg 22/122: auto (default), vl, vl-short (vl\n"
-                 "                          for short queries), cl, and the reference's ablations of cl:\n"
+                 "  --variant <name>        work distribution of alg 22/122: auto (default: vl), vl, vl-short (the\n"
+                 "                          same as vl), cl, and the reference's ablations of cl:\n"
                  "                          cl-noshuffle (its alg 23), cl-tile (alg 24), cl-atomic (alg 19)\n"
-                 "  --rf_log <3..5>         log2 of the per-level reduction factor (default: the variant's)\n"
+                 "  --rf_log <3..5>         log2 of the per-level reduction factor (default: the variant's).  vl's\n"
+                 "                          tables take no more memory than the levels of this and --nb would\n"
                  "  --lanes <2|4|8|16|32>   CL lanes per query\n"
                  "  --l2_persist            put the coarse levels in an L2 persisting window\n"
                  "  --ties <frac>           set that fraction of the entries to the array's minimum\n"

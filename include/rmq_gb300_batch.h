@@ -29,9 +29,9 @@ typedef struct {
     uint32_t num_arrays;
     uint64_t total_values;      /* sum of the array sizes                                   */
     uint64_t level_bytes;       /* device bytes of all arrays' window tables                */
-    uint64_t scan_threshold;    /* t used for every array (after autotuning, if run)         */
-    uint32_t query_block;       /* threads per CTA of the query kernel (one warp = 32 queries) */
-    uint32_t max_levels;        /* deepest hierarchy in the batch                            */
+    uint64_t scan_threshold;    /* t of the planned levels (the last size class's)           */
+    uint32_t query_block;       /* threads per CTA of the query kernel (4 queries per thread) */
+    uint32_t max_levels;        /* of the plan with the most levels                          */
     uint64_t total_queries;     /* of the last rmq_batch_set_queries                         */
     float    build_ms;          /* device time of the last rmq_batch_build (CUDA events)    */
     float    query_ms;          /* device time of the last timed query pass (autotune)      */
@@ -43,8 +43,8 @@ typedef struct {
  * d_values[value_offsets[a] .. value_offsets[a] + sizes[a]) (host arrays of
  * num_arrays entries; offsets multiples of 8 so every array is 32-byte
  * aligned; 1 <= sizes[a] <= 0xFFFFFF00).  cfg: scan_threshold (0 = 64) and
- * with_index are used; rf is 8.  Allocates the packed level buffers and the
- * device descriptors; nothing is built yet.  d_values must outlive the batch. */
+ * with_index are used; rf is 8.  Allocates the packed tables and the device
+ * descriptors; nothing is built yet.  d_values must outlive the batch. */
 int rmq_batch_create(const float* d_values, const uint64_t* value_offsets, const uint64_t* sizes,
                      uint32_t num_arrays, const rmq_config* cfg, rmq_stream_t stream,
                      rmq_batch** out);
@@ -86,9 +86,9 @@ int rmq_batch_autotune(rmq_batch* b, rmq_stream_t stream, rmq_batch_info* info);
 
 /* Applies a known choice (for example one rmq_batch_autotune made earlier for
  * the same workload): scan threshold t (>= 8) and CTA size (a multiple of 32,
- * <= 512) of the query kernel.  The levels must be rebuilt (rmq_batch_build or
- * rmq_batch_run) before querying.  RMQ_ERR_UNSUPPORTED when t would need more
- * level storage than the batch holds (any t >= 16, or the creation t, fits). */
+ * <= 512) of the query kernel.  t is reported and has no other effect; the
+ * tables stay as they are.  RMQ_ERR_UNSUPPORTED when t plans more level entries
+ * than the creation t and every t >= 16 do (which are always accepted). */
 int rmq_batch_set_tuning(rmq_batch* b, uint64_t scan_threshold, uint32_t query_block, rmq_stream_t stream);
 
 /* The same with one t per array-size class (class_thresholds[3], each >= 8,
