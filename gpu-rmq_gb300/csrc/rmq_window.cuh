@@ -719,16 +719,17 @@ __device__ __forceinline__ WinBest<I> win_short_once(const WinViewT<I>& w, I l, 
 }
 
 // The part [x, y) of a query [l, R) that lies on whole strides of 2^gb: true
-// when it holds eight of them, so that windows inside the query serve it.
-// Within eight strides of 2^32 sums with x wrap, and x itself within one of
-// 2^9, so the distance decides: y - x is no more than the query's length just
-// where neither x nor the difference has wrapped.
-template <typename I>
+// when it holds eight of them, so that windows inside the query serve it.  With
+// 32-bit positions the distance decides, since x plus eight strides would wrap
+// near 2^32; x itself does for l above 2^32 - 2^9 with the strides of 2^9 that only tables with LARGE
+// blocks have (n goes up to 2^32 - 2^8).
+template <bool LARGE, typename I>
 __host__ __device__ __forceinline__ bool win_inner(I l, I R, uint32_t gb, I& x, I& y) {
     const I gm = (I(1) << gb) - 1u;
     x = (l + gm) & ~gm;
     y = R & ~gm;
-    return y - x <= R - l && y - x >= (I(8) << gb);
+    if (sizeof(I) == 8) return y >= x + (I(8) << gb);
+    return (!LARGE || x >= l) && y >= x && y - x >= (I(8) << gb);
 }
 
 // The exact answer of [l, R) from entries inside it, for a query whose cover
@@ -745,13 +746,13 @@ __host__ __device__ __forceinline__ bool win_inner(I l, I R, uint32_t gb, I& x, 
 // left of l; in the first sector of V1 already for three in five where one
 // value in 100 is the minimum: the mixture of lengths with n = 2^28, q = 2^27
 // 4858 -> 4801 us).
-template <typename I>
+template <bool LARGE, typename I>
 __device__ __forceinline__ void win_exact(const WinViewT<I>& w, I l, I R, float bound, WinBest<I>& cur, float& vl,
                                           float& vr) {
     const uint32_t gb = w.gb, step = w.c;
     const I bl = l >> w.blk, br = (R - 1u) >> w.blk, last = br & ~I(7);
     I x, y;
-    const bool windows = win_inner(l, R, gb, x, y);
+    const bool windows = win_inner<LARGE>(l, R, gb, x, y);
     const I by = y >> w.blk;
     I b = bl & ~I(7);
     {
@@ -1068,7 +1069,7 @@ __device__ __forceinline__ uint32_t win_block(const WinViewT<I>& w, const WinLis
         const I l = q.x, R = q.y + 1u;
         WinBest<I> c = win_none<I>();
         float vl = f_inf(), vr = f_inf();
-        win_exact(w, l, R, sm.bound[t], c, vl, vr);
+        win_exact<LARGE>(w, l, R, sm.bound[t], c, vl, vr);
         win_ends<LARGE>(w, l, R, vl, vr, c);
         store(c, l, slot);
     }
@@ -1094,7 +1095,7 @@ __device__ __forceinline__ WinBest<I> win_one(const WinViewT<I>& w, I l, I r) {
     if (!LARGE && (len >> w.first) == 0u) return w.blk == 3u ? win_short_once<1>(w, l, R) : win_short_once<2>(w, l, R);
     WinBest<I> c = win_none<I>();
     float vl = f_inf(), vr = f_inf();
-    win_exact(w, l, R, bound, c, vl, vr);
+    win_exact<LARGE>(w, l, R, bound, c, vl, vr);
     win_ends<LARGE>(w, l, R, vl, vr, c);
     return c;
 }

@@ -18,9 +18,12 @@ static void check(const WinView& w32, const WinView64& w64, uint64_t l, uint64_t
     ++checked;
     uint32_t x32, y32;
     uint64_t x64, y64;
-    const bool a = win_inner(uint32_t(l), uint32_t(R), w32.gb, x32, y32);
-    const bool b = win_inner(l, R, w64.gb, x64, y64);
-    if (a != b || (a && (x32 != x64 || y32 != y64))) report("inner", l, R);
+    const bool large = w32.blk > 4;
+    const bool a = large ? win_inner<true>(uint32_t(l), uint32_t(R), w32.gb, x32, y32)
+                         : win_inner<false>(uint32_t(l), uint32_t(R), w32.gb, x32, y32);
+    const bool b = win_inner<true>(l, R, w64.gb, x64, y64);
+    if (a != b || (a && (x32 != x64 || y32 != y64 || y64 < x64 || y64 - x64 < uint64_t(8) << w64.gb)))
+        report("inner", l, R);
     const uint64_t len = R - l;
     if ((len >> (w32.first - 1u)) == 0) return;
     uint32_t k32, k64, s1, s2;
