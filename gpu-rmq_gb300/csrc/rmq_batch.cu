@@ -64,7 +64,7 @@ batch_top_kernel(const ArrayDesc* __restrict__ descs, TileList l, char* tables) 
     __shared__ uint2 sa[kTopEntries], sb[kTopEntries / 2];
     WinOut w;
     batch_tile(descs, l, nullptr, tables, w);
-    win_top(w, sa, sb);
+    win_top(w, win_mid_log(w), sa, sb);
 }
 
 // Work unit of the query kernels: consecutive queries of one array, answered by
@@ -568,6 +568,7 @@ int rmq_batch_run_per_array(rmq_batch* b, rmq_stream_t stream) {
         qa.q = q;
         qa.out_min = b->d_min != nullptr ? b->d_min + q0 : nullptr;
         qa.out_idx = b->d_argmin != nullptr ? b->d_argmin + q0 : nullptr;
+        qa.after_build = true;
         qa.variant = RMQ_VARIANT_VL;
         qa.rf_log = 3;
         e = rmq::launch_query(qa, s);

@@ -39,8 +39,9 @@ uint64_t tail_counters(const Layout& lay);
 cudaError_t launch_window_build(const float* d_values, void* tables, uint64_t n, uint32_t form, bool wide,
                                 cudaStream_t s);
 // Loads the code of every kernel that a build of kFormArgmin with 32-bit
-// positions and its queries can launch, on the current device.
-cudaError_t load_window_kernels();
+// positions over up to kSmallN values and its queries can launch, on the current
+// device.
+cudaError_t load_small_window_kernels();
 
 struct QueryArgs {
     Levels lv;
@@ -49,6 +50,7 @@ struct QueryArgs {
     float* out_min;      // may be null for argmin queries
     uint32_t* out_idx;   // null for min queries
     WinView win;         // VL: the window tables (lv is CL's)
+    bool after_build;    // the build was launched just before, on the same stream
     bool host_buffers;   // queries and results in host memory, over the CPU-GPU link
     bool wide;           // 64-bit positions: win64 / qs64 / out_idx64 are used instead
     WinView64 win64;
@@ -126,7 +128,9 @@ struct ServeQueryArgs {
 cudaError_t launch_serve_query(const ServeQueryArgs& a, cudaStream_t s);
 cudaError_t launch_fill_owner(const uint64_t* unit_off, uint32_t num, uint32_t* owner, cudaStream_t s);
 
-// Kernel launch with the handle's L2 access-policy window, when it has one.
+// Kernel launch with the handle's L2 access-policy window, when it has one, or,
+// after a build without one, scheduled before the build's last kernel ends (for
+// kernels that wait for it themselves).
 template <typename K, typename... Args>
 static cudaError_t launch_with_window(K kernel, uint32_t grid, uint32_t block, const QueryArgs& a,
                                       cudaStream_t s, Args... args) {
@@ -136,7 +140,12 @@ static cudaError_t launch_with_window(K kernel, uint32_t grid, uint32_t block, c
     cfg.dynamicSmemBytes = 0;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
-    if (a.persist_base != nullptr && a.persist_bytes > 0) {
+    if (a.after_build) {
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    } else if (a.persist_base != nullptr && a.persist_bytes > 0) {
         attr[0].id = cudaLaunchAttributeAccessPolicyWindow;
         attr[0].val.accessPolicyWindow.base_ptr = const_cast<void*>(a.persist_base);
         attr[0].val.accessPolicyWindow.num_bytes = a.persist_bytes;

@@ -95,7 +95,7 @@ int scratch_for_current_device(void** out) {
             cudaGetLastError();
             return RMQ_ERR_CUDA;
         }
-        if (rmq::load_window_kernels() != cudaSuccess) {
+        if (rmq::load_small_window_kernels() != cudaSuccess) {
             cudaGetLastError();
             return RMQ_ERR_CUDA;
         }
@@ -129,7 +129,11 @@ extern "C" int rmq_query_idx_static(const float* d_values, uint64_t n, uint64_t 
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
 
     // Every table entry a query reads is rewritten by the build of this call, so nothing
-    // in the scratch needs clearing between calls.
+    // in the scratch needs clearing between calls.  Up to 2^18 queries their kernel is
+    // scheduled while the build ends.  256 queries of lognormal(2^13, 1), us a call,
+    // n = 1000, 2^14, 2^17, 2^20, 2^22: 5.5, 9.4, 12.6, 14.5, 20.6 (build and queries
+    // one after the other, by the build kernels for large arrays: 10.5, 14.5, 18.6,
+    // 20.7, 28.7; on block-minimum levels 8.6, 12.4, 12.6, 16.5, 18.6).
     cudaError_t e = rmq::launch_window_build(d_values, scratch, n, rmq::kFormArgmin, false, s);
     if (e == cudaSuccess && q > 0) {
         rmq::QueryArgs a;
@@ -139,6 +143,7 @@ extern "C" int rmq_query_idx_static(const float* d_values, uint64_t n, uint64_t 
         a.q = q;
         a.out_min = d_min_or_null;
         a.out_idx = d_argmin;
+        a.after_build = true;
         a.variant = RMQ_VARIANT_VL;
         a.rf_log = kStaticRfLog;
         e = rmq::launch_query(a, s);

@@ -33,10 +33,17 @@ __global__ void __launch_bounds__(kMidThreads) win_mid_kernel(WinOut w) {
     win_mid_tile(w, blockIdx.x, sa, sb);
 }
 
-__global__ void __launch_bounds__(kMidThreads) win_top_kernel(WinOut w) {
+__global__ void __launch_bounds__(kMidThreads) win_top_kernel(WinOut w, uint32_t k0) {
     __shared__ uint2 sa[kTopEntries], sb[kTopEntries / 2];
     wait_previous_grid();
-    win_top(w, sa, sb);
+    win_top(w, k0, sa, sb);
+}
+
+template <uint32_t HALO>
+__global__ void __launch_bounds__(win_small_threads<HALO>()) win_small_kernel(WinOut w) {
+    __shared__ WinSmallShared<HALO> sm;
+    allow_next_grid();
+    win_small_tile<HALO>(w, blockIdx.x, sm);
 }
 
 // Launch with programmatic stream serialization (the kernel waits for its
@@ -74,13 +81,23 @@ cudaError_t launch_window_build(const float* d_values, void* tables, uint64_t n,
     w.first = sh.first;
     w.kmax = sh.kmax;
     w.wide = wide;
+    if (n <= kSmallN && sh.gb == 5u) {
+        const bool brief = n <= kShortHaloN && (sh.S <= kShortHalo || sh.S > kLongHalo);
+        const uint64_t halo = brief ? kShortHalo : kLongHalo;
+        const uint32_t tiles = uint32_t((sh.S + halo - 1) / halo), k0 = sh.gb + (brief ? 7u : 9u);
+        if (brief) win_small_kernel<kShortHalo><<<tiles, win_small_threads<kShortHalo>(), 0, s>>>(w);
+        else win_small_kernel<kLongHalo><<<tiles, win_small_threads<kLongHalo>(), 0, s>>>(w);
+        const cudaError_t e = cudaGetLastError();
+        return e != cudaSuccess || tiles == 1 || sh.kmax <= k0 ? e
+                                                               : launch_dependent(win_top_kernel, 1u, kMidThreads, s, w, k0);
+    }
     const WinTiles t = win_tiles(sh);
     (sh.blk > 4u ? win_block_kernel<true> : win_block_kernel<false>)<<<uint32_t(t.block), kBlockThreads, 0, s>>>(w);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess && t.low > 0) e = launch_dependent(sh.gb - sh.blk == 3u ? win_low_kernel<true> : win_low_kernel<false>,
                                                         uint32_t(t.low), kLowThreads, s, w);
     if (e == cudaSuccess && t.mid > 0) e = launch_dependent(win_mid_kernel, uint32_t(t.mid), kMidThreads, s, w);
-    if (e == cudaSuccess && t.top > 0) e = launch_dependent(win_top_kernel, uint32_t(t.top), kMidThreads, s, w);
+    if (e == cudaSuccess && t.top > 0) e = launch_dependent(win_top_kernel, uint32_t(t.top), kMidThreads, s, w, win_mid_log(sh));
     return e;
 }
 
@@ -136,6 +153,10 @@ template <bool ARGMIN, typename I, bool LARGE = false>
 __global__ void __launch_bounds__(kOneThreads)
 win_one_kernel(WinViewT<I> w, const typename IdxTraits<I>::Pair* __restrict__ qs, uint64_t q,
                float* __restrict__ out_min, I* __restrict__ out_idx, uint32_t* __restrict__ err) {
+    // After a build (QueryArgs::after_build) its last kernel may still run.  The
+    // loads are not volatile, and all depend on a query's: its address comes
+    // from the wait, so none can move before it.
+    asm volatile("griddepcontrol.wait;" : "+l"(qs) : : "memory");
     using C = typename IdxTraits<I>::Count;
     const C i = C(blockIdx.x) * kOneThreads + threadIdx.x;
     if (uint64_t(blockIdx.x) * kOneThreads + threadIdx.x >= q) return;
@@ -171,10 +192,12 @@ static cudaError_t launch_window_typed(const QueryArgs& a, const WinViewT<I>& w,
         return launch_with_window(large ? win_one_kernel<ARGMIN, I, true> : win_one_kernel<ARGMIN, I>,
                                   uint32_t((a.q + kOneThreads - 1u) / kOneThreads), kOneThreads, a, s, w, qs, a.q,
                                   a.out_min, out_idx, a.err);
+    QueryArgs plain = a;  // the block kernel does not wait for a build
+    plain.after_build = false;
     return launch_with_window(large             ? win_query_kernel<ARGMIN, true, I, true>
                               : w.n > kWarmN    ? win_query_kernel<ARGMIN, true, I>
                                                 : win_query_kernel<ARGMIN, false, I>,
-                              uint32_t((a.q + kBlockQueries - 1u) / kBlockQueries), kQueryThreads, a, s, w, qs, a.q,
+                              uint32_t((a.q + kBlockQueries - 1u) / kBlockQueries), kQueryThreads, plain, s, w, qs, a.q,
                               a.out_min, out_idx, a.err);
 }
 
@@ -190,14 +213,12 @@ cudaError_t launch_window_query(const QueryArgs& a, cudaStream_t s) {
 
 // The runtime loads a kernel's code with its first launch unless something
 // asks for its attributes before.
-cudaError_t load_window_kernels() {
-    const void* const kernels[] = {reinterpret_cast<const void*>(&win_block_kernel<false>),
-                                   reinterpret_cast<const void*>(&win_low_kernel<false>),
-                                   reinterpret_cast<const void*>(&win_mid_kernel),
+cudaError_t load_small_window_kernels() {
+    const void* const kernels[] = {reinterpret_cast<const void*>(&win_small_kernel<kShortHalo>),
+                                   reinterpret_cast<const void*>(&win_small_kernel<kLongHalo>),
                                    reinterpret_cast<const void*>(&win_top_kernel),
                                    reinterpret_cast<const void*>(&win_one_kernel<true, uint32_t>),
-                                   reinterpret_cast<const void*>(&win_query_kernel<true, false, uint32_t>),
-                                   reinterpret_cast<const void*>(&win_query_kernel<true, true, uint32_t>)};
+                                   reinterpret_cast<const void*>(&win_query_kernel<true, false, uint32_t>)};
     for (const void* k : kernels) {
         cudaFuncAttributes at;
         const cudaError_t e = cudaFuncGetAttributes(&at, k);

@@ -2,11 +2,12 @@
 // the single-array kernels (rmq_window.cu) and the batched ones (rmq_batch.cu).
 //
 // One streaming pass over level 0 writes the minimum and its offset for every
-// block (0.31 n bytes with blocks of 16 entries); everything above is computed from those,
-// which are still in L2.  A tile pass holds 2048 strides and a halo of 512 in
-// shared memory and makes every table whose windows fit the halo; a second
-// tile pass does the same for the next six sizes; one CTA makes the few
-// entries above.  Each table is one doubling of the one below:
+// block (0.31 n bytes with blocks of 16 entries); everything above is computed
+// from those, which are still in L2.  A tile pass holds 2048 strides and a halo
+// of 512 in shared memory and makes every table whose windows fit the halo; a
+// second tile pass does the same for the next six sizes; one CTA makes the few
+// entries above.  Small arrays take smaller tiles, straight from level 0, and
+// that last CTA.  Each table is one doubling of the one below:
 // T_(k+1)[i] = first minimum of T_k[2i] and T_k[2i + windows per stride].
 #pragma once
 
@@ -21,7 +22,7 @@ constexpr uint32_t kMidThreads = 1024;
 constexpr uint32_t kSpan = 2048;           // own strides per tile of the window kernels
 constexpr uint32_t kHaloLow = 512;         // halo of the first window kernel, in strides of 2^gb
 constexpr uint32_t kHaloMid = 1024;        // halo of the second, in its input's strides
-constexpr uint32_t kTopEntries = 4096;     // entries of T_(gb+15) the last kernel holds in shared memory
+constexpr uint32_t kTopEntries = 4096;     // entries the last kernel holds in shared memory
 constexpr uint32_t kMidSteps = 6;          // sizes the second window kernel adds
 
 // Largest window the first kernel makes from a tile and its halo (512 strides
@@ -31,19 +32,19 @@ __host__ __device__ __forceinline__ uint32_t win_low_log(const V& w) { return w.
 template <typename V>
 __host__ __device__ __forceinline__ uint32_t win_mid_log(const V& w) { return w.gb + 9u + kMidSteps; }
 
-// Blocks of one tile.  A warp's load covers 32 consecutive sectors (1 KiB);
-// each lane takes its sector's first minimum, and the two lanes of a block
-// exchange one sector each of two loads, so that every lane ends with one
-// whole block and a warp stores 32 consecutive blocks.  LARGE: blocks of 32 or
-// 64 entries, four or eight lanes each.
-template <bool LARGE>
-__device__ __forceinline__ void win_block_tile(const WinOut& w, uint64_t tile) {
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint64_t base = tile * kBlockTile;
-    const uint64_t sec0 = (base >> 3) + warp * 128u + lane;
+// Blocks of a warp's 1024 values from `base`, handed to put(block, minimum,
+// offset).  A load covers 32 consecutive sectors (1 KiB); each lane takes its
+// sector's first minimum, and the two lanes of a block exchange one sector each
+// of two loads, so that every lane ends with one whole block and a warp stores
+// 32 consecutive blocks.  LARGE: blocks of 32 or 64 entries, four or eight lanes
+// each.
+template <bool LARGE, typename Put>
+__device__ __forceinline__ void win_block_part(const WinOut& w, uint64_t base, const Put& put) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t sec0 = (base >> 3) + lane;
     const uint64_t pol = policy_evict_first();
     float v[4][8];
-    if (base + kBlockTile <= w.n) {
+    if (base + 1024u <= w.n) {
 #pragma unroll
         for (uint32_t i = 0; i < 4; ++i) ld_sector_policy(w.a + 8u * (sec0 + 32u * i), v[i], pol);
     } else {
@@ -90,10 +91,7 @@ __device__ __forceinline__ void win_block_tile(const WinOut& w, uint64_t tile) {
                 }
             }
             const uint64_t sec = sec0 + 32u * i;
-            if ((lane & (sectors - 1u)) == 0u && (sec << 3) < w.n) {
-                w.v1[sec >> (w.blk - 3u)] = m[i];
-                w.j1[sec >> (w.blk - 3u)] = uint8_t(off[i]);
-            }
+            if ((lane & (sectors - 1u)) == 0u && (sec << 3) < w.n) put(sec >> (w.blk - 3u), m[i], off[i]);
         }
         return;
     }
@@ -101,10 +99,7 @@ __device__ __forceinline__ void win_block_tile(const WinOut& w, uint64_t tile) {
 #pragma unroll
         for (uint32_t i = 0; i < 4; ++i) {
             const uint64_t blk = sec0 + 32u * i;
-            if ((blk << 3) < w.n) {
-                w.v1[blk] = m[i];
-                w.j1[blk] = uint8_t(off[i]);
-            }
+            if ((blk << 3) < w.n) put(blk, m[i], off[i]);
         }
         return;
     }
@@ -119,11 +114,17 @@ __device__ __forceinline__ void win_block_tile(const WinOut& w, uint64_t tile) {
         const uint32_t loo = odd ? oo : mo, hio = odd ? mo : oo;
         const bool hi = hiv < lov;  // equal: the first sector's entry stays
         const uint64_t blk = (sec0 + 32u * (odd ? p + 1u : p)) >> 1;
-        if ((blk << 4) < w.n) {
-            w.v1[blk] = hi ? hiv : lov;
-            w.j1[blk] = uint8_t(hi ? 8u + hio : loo);
-        }
+        if ((blk << 4) < w.n) put(blk, hi ? hiv : lov, hi ? 8u + hio : loo);
     }
+}
+
+// Blocks of one tile, by kBlockThreads threads.
+template <bool LARGE>
+__device__ __forceinline__ void win_block_tile(const WinOut& w, uint64_t tile) {
+    win_block_part<LARGE>(w, tile * kBlockTile + (threadIdx.x >> 5) * 1024u, [&](uint64_t blk, float m, uint32_t off) {
+        w.v1[blk] = m;
+        w.j1[blk] = uint8_t(off);
+    });
 }
 
 // First minimum of two entries; hi_off: what the upper one's offset gains (0
@@ -206,21 +207,21 @@ __device__ __forceinline__ uint2 win_group(const WinOut& w, uint64_t g) {
     return e;
 }
 
-// The tables up to T_(gb+9) (all of them when the array has one tile) of the
-// tile's kSpan strides of 2^gb entries, by kLowThreads threads.  A tile is a
-// chain of some ten steps with a barrier each, so its time is their latency:
-// every thread keeps its entries in registers, all loads of a step in flight
-// (one tile: 16 -> 8.5 us against one entry after another with 256 threads;
-// the build of 2^20 values 25 -> 19 us, of 2^26 80 -> 71 us).
-template <bool EIGHT>
-__device__ __forceinline__ void win_low_tile(const WinOut& w, uint64_t tile, uint2* sa, uint2* sb) {
-    constexpr uint32_t kPer = (kSpan + kHaloLow) / kLowThreads;
-    const uint64_t g0 = tile * kSpan;
+// The tables up to T_(gb + log2 HALO) (all of them when the array has one tile)
+// of a tile's SPAN strides from g0, by THREADS threads; group(i, g): the entry
+// of stride g, the tile's i-th.  A tile is a chain of some ten steps with a
+// barrier each, so its time is their latency: every thread keeps its entries in
+// registers, all loads of a step in flight (one tile of kSpan strides: 16 ->
+// 8.5 us against one entry after another with 256 threads).
+template <uint32_t SPAN, uint32_t HALO, uint32_t THREADS, typename Group>
+__device__ __forceinline__ void win_tile_tables(const WinOut& w, uint64_t g0, uint32_t top, uint2* sa, uint2* sb,
+                                                const Group& group) {
+    constexpr uint32_t kPer = (SPAN + HALO) / THREADS;
     uint2 e[kPer];
 #pragma unroll
     for (uint32_t u = 0; u < kPer; ++u) {
-        const uint64_t g = g0 + threadIdx.x + kLowThreads * u;
-        if (g < w.S) e[u] = win_group<EIGHT>(w, g);
+        const uint64_t g = g0 + threadIdx.x + THREADS * u;
+        if (g < w.S) e[u] = group(threadIdx.x + THREADS * u, g);
     }
     // Windows of 2, 4, 8 strides (2^first entries), the last one the first
     // table; where the next one has the same stride, a doubling of 8.
@@ -228,7 +229,7 @@ __device__ __forceinline__ void win_low_tile(const WinOut& w, uint64_t tile, uin
     const uint32_t kb = w.gb + w.c;
     for (uint32_t d = 1;; d <<= 1) {
 #pragma unroll
-        for (uint32_t u = 0; u < kPer; ++u) src[threadIdx.x + kLowThreads * u] = e[u];
+        for (uint32_t u = 0; u < kPer; ++u) src[threadIdx.x + THREADS * u] = e[u];
         __syncthreads();
         if (d > (w.first < kb ? 8u : 4u)) break;
         uint2* out = nullptr;
@@ -236,17 +237,79 @@ __device__ __forceinline__ void win_low_tile(const WinOut& w, uint64_t tile, uin
         if (d == 8u && w.kmax >= kb) out = w.t + win_table_at<uint64_t>(w, kb) + g0;
 #pragma unroll
         for (uint32_t u = 0; u < kPer; ++u) {
-            const uint32_t i = threadIdx.x + kLowThreads * u;
-            if (g0 + i + d < w.S && i + d < kSpan + kHaloLow) e[u] = win_first(e[u], src[i + d], w.wide ? d << w.gb : 0u);
-            if (out != nullptr && i < kSpan && g0 + i < w.S) out[i] = e[u];
+            const uint32_t i = threadIdx.x + THREADS * u;
+            if (g0 + i + d < w.S && i + d < SPAN + HALO) e[u] = win_first(e[u], src[i + d], w.wide ? d << w.gb : 0u);
+            if (out != nullptr && i < SPAN && g0 + i < w.S) out[i] = e[u];
         }
         uint2* x = src;
         src = dst;
         dst = x;
     }
-    const uint32_t last = w.S <= kSpan ? w.kmax : (w.kmax < win_low_log(w) ? w.kmax : win_low_log(w));
-    win_double_up(w, kb, last, g0, kSpan + kHaloLow, kSpan, src, dst);
+    const uint32_t last = w.S <= SPAN ? w.kmax : (w.kmax < top ? w.kmax : top);
+    win_double_up(w, kb, last, g0, SPAN + HALO, SPAN, src, dst);
 }
+
+// The tables up to T_(gb+9) of one tile, from V1 and J1.
+template <bool EIGHT>
+__device__ __forceinline__ void win_low_tile(const WinOut& w, uint64_t tile, uint2* sa, uint2* sb) {
+    win_tile_tables<kSpan, kHaloLow, kLowThreads>(w, tile * kSpan, win_low_log(w), sa, sb,
+                                                  [&](uint32_t, uint64_t g) { return win_group<EIGHT>(w, g); });
+}
+
+// Small arrays (kFormArgmin and kFormSmallMin, up to kSmallN entries) are built
+// by one kernel from level 0 and, above one tile, one CTA for the sizes above:
+// what such a build costs is its launches and the chain of steps in each, not
+// bytes.  A tile is HALO strides of 32 values of its own and as many behind
+// them, whose blocks it computes again: 128 keep the chain short, but leave
+// n / 2^8 entries to the last CTA, which holds 4096, so above 2^20 values (and
+// for the one tile of 2^12 to 2^14) it is 512.  Device time of rmq_build for
+// 1000, 2^14, 2^18, 2^20 and 2^22 values, us: 10.5, 11.9, 14.6, 16.2 and 20.6; with
+// the kernels for large arrays 13.8, 14.9, 19.4, 20.7 and 23.1; the block-minimum
+// levels took 11.1, 11.1, 13.4, 14.1 and 17.8.
+constexpr uint64_t kShortHaloN = uint64_t(1) << 20;
+constexpr uint32_t kShortHalo = 128, kLongHalo = 512;
+template <uint32_t HALO>
+__host__ __device__ constexpr uint32_t win_small_threads() { return HALO == kShortHalo ? 256u : 512u; }
+
+template <uint32_t HALO>
+struct WinSmallShared {
+    float v1[8 * HALO];  // up to four blocks per stride
+    uint8_t j1[8 * HALO];
+    uint2 a[2 * HALO], b[2 * HALO];
+};
+
+template <uint32_t HALO>
+__device__ __forceinline__ void win_small_tile(const WinOut& w, uint64_t tile, WinSmallShared<HALO>& sm) {
+    constexpr uint32_t kThreads = win_small_threads<HALO>(), kWarps = kThreads / 32u;
+    const uint64_t g0 = tile * HALO;
+    const uint32_t bpg = 1u << (w.gb - w.blk);  // blocks per stride: 2 or 4
+    const uint64_t b0 = g0 * bpg, nb = (w.n + (uint64_t(1) << w.blk) - 1) >> w.blk;
+#pragma unroll 1
+    for (uint32_t part = threadIdx.x >> 5; part < HALO / 16u; part += kWarps) {  // 32 strides a part
+        const uint64_t base = (g0 << w.gb) + part * 1024u;
+        if (base >= w.n) break;
+        win_block_part<false>(w, base, [&](uint64_t blk, float m, uint32_t off) {
+            const uint32_t i = uint32_t(blk - b0);
+            sm.v1[i] = m;
+            sm.j1[i] = uint8_t(off);
+            if (i < HALO * bpg) {
+                w.v1[blk] = m;
+                w.j1[blk] = uint8_t(off);
+            }
+        });
+    }
+    if (w.n < (uint64_t(1) << w.first)) return;
+    __syncthreads();
+    win_tile_tables<HALO, HALO, kThreads>(w, g0, w.gb + (HALO == kShortHalo ? 7u : 9u), sm.a, sm.b, [&](uint32_t i, uint64_t g) {
+        const uint32_t b = i * bpg;
+        uint2 e = make_uint2(__float_as_uint(sm.v1[b]), sm.j1[b]);
+        for (uint32_t c = 1; c < bpg && g * bpg + c < nb; ++c)
+            e = win_first(e, make_uint2(__float_as_uint(sm.v1[b + c]), sm.j1[b + c]), c << w.blk);
+        if (!w.wide) e.y += uint32_t(g << w.gb);
+        return e;
+    });
+}
+
 
 // The next kMidSteps tables above T_(gb+9) of one tile of its entries.
 __device__ __forceinline__ void win_mid_tile(const WinOut& w, uint64_t tile, uint2* sa, uint2* sb) {
@@ -284,11 +347,11 @@ inline WinTiles win_tiles(const WinShape& w) {
     return t;
 }
 
-// The tables above T_(gb+15), by one CTA of kMidThreads: from shared memory
-// where its entries fit there (up to 2^28 entries), else each table from the
-// one below in global memory.
-__device__ __forceinline__ void win_top(const WinOut& w, uint2* sa, uint2* sb) {
-    const uint32_t k0 = win_mid_log(w), s0 = win_stride_log(w, k0);
+// The tables above T_k0, by one CTA of kMidThreads: from shared memory where its
+// entries fit there (k0 = win_mid_log: up to 2^28 values), else each table from
+// the one below in global memory.
+__device__ __forceinline__ void win_top(const WinOut& w, uint32_t k0, uint2* sa, uint2* sb) {
+    const uint32_t s0 = win_stride_log(w, k0);
     const uint64_t have = (w.n + (uint64_t(1) << s0) - 1) >> s0;
     const uint2* from = w.t + win_table_at<uint64_t>(w, k0);
     if (have <= kTopEntries) {
