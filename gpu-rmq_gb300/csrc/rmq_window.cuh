@@ -1,8 +1,8 @@
 // rmq_window.cuh — the window tables and the query over them.
 //
 // What bounds a query is the number of random sectors it reads: an SM looks up
-// one 128-byte line per cycle (289 G lines/s over the chip, measured with
-// random 4- to 16-byte loads that hit L2) and DRAM serves about 46 G random
+// one 128-byte line per cycle (289 to 302 G lines/s over the chip by box, measured
+// with random 4- to 16-byte loads of 16 MiB) and DRAM serves about 46 G random
 // lines/s, so a level-by-level descent that reads ten sectors per query, two
 // of them at level 0 in DRAM, ends near 26 G queries/s however it is
 // scheduled.  The tables cut both counts: a long query reads two 8-byte
